@@ -15,6 +15,7 @@
 #include <cstdint>
 
 #include "exp_table.h"
+#include "intpath.cuh"
 #include "stream.h"
 
 namespace stg {
@@ -26,6 +27,10 @@ struct PState {
     // policy, refreshed whenever rvv changes: chi charge_ratio (e q0)^2
     // (1 - beta0 beta) / (pc0 beta) and 1 / rvv (pc0 = p0c e, beta = beta0 rvv)
     double sc_k, inv_rvv;
+    // (rvv - 1) 2^53 and the range limit of the drift's integer path
+    // (intpath.cuh drift_slip), refreshed with them
+    int64_t rvv53;
+    uint32_t slip_lim;
     int64_t pid, at_element, at_turn, state;
     bool lazy_s;    // s is +0 at this turn's start: s is read from the lattice's s table
 };
@@ -93,6 +98,8 @@ __device__ __forceinline__ void refresh_kick_factors(PState &p)
     double const charge = kCharge0SiD * p.q0;
     p.sc_k = p.chi * p.charge_ratio * charge * charge * (1.0 - p.beta0 * beta) * inv_pc0_beta;
     p.inv_rvv = inv_pc0_beta * (pc0 * p.beta0);
+    p.rvv53 = slip_rvv(p.rvv);
+    p.slip_lim = slip_limit(p.rvv);
 }
 
 // ------------------------------------------------------------------ energy
@@ -145,10 +152,24 @@ __device__ __forceinline__ void add_s(PState &p, double L)
     }
 }
 
+// rvv - (1 + (xp^2 + yp^2) / 2) on the FP64 pipe, for the lanes the integer
+// path leaves undecided (out of line: predicated-off FP64 instructions
+// would occupy the pipe for every drift).
+template <bool FAST>
+static __device__ __noinline__ double drift_slip_fp64(double xp, double yp, double rvv)
+{
+    if (FAST) return rvv - fma(fma(yp, yp, xp * xp), 0.5, 1.0);
+    return rvv - (1.0 + (xp * xp + yp * yp) * 0.5);
+}
+
+static __device__ __noinline__ double drift_slip_large(int64_t v) { return scaled_53_large(v); }
+
 // be_drift/track.h:45-67.  FAST keeps the reference's rounding of
-// 1 + (xp^2 + yp^2)/2 at the scale of 1.0 (u below): regrouping the zeta
-// update as L (rvv - 1) - (L/2)(xp^2 + yp^2) is more accurate but departs
-// from the reference by its own rounding noise, ~1e-16 m per drift.
+// 1 + (xp^2 + yp^2)/2 at the scale of 1.0: regrouping the zeta update as
+// L (rvv - 1) - (L/2)(xp^2 + yp^2) is more accurate but departs from the
+// reference by its own rounding noise, ~1e-16 m per drift.  The slip
+// rvv - (1 + (xp^2 + yp^2)/2) comes from the integer pipe with the FP64
+// sequence's bits (drift_slip).
 // s is only accumulated when the turn did not start at s = +0 (otherwise it
 // comes from the lattice's s table).
 template <bool FAST, bool S_LIVE = true>
@@ -157,16 +178,23 @@ __device__ __forceinline__ void drift(PState &p, double L)
     double const xp = p.px * p.rpp;
     double const yp = p.py * p.rpp;
     if (FAST) {
-        double const u = fma(fma(yp, yp, xp * xp), 0.5, 1.0);
         p.x = fma(xp, L, p.x);
         p.y = fma(yp, L, p.y);
-        p.zeta = fma(L, p.rvv - u, p.zeta);
     } else {
-        double const dzeta = p.rvv - (1.0 + (xp * xp + yp * yp) * 0.5);
         p.x += xp * L;
         p.y += yp * L;
-        p.zeta += L * dzeta;
     }
+    int64_t slip53;
+    bool const known = drift_slip(xp, yp, p.rvv53, p.slip_lim, &slip53);
+    double dzeta = scaled_53(slip53);
+    if (!known)
+        dzeta = drift_slip_fp64<FAST>(xp, yp, p.rvv);
+    else if (!below_2_32(slip53))
+        dzeta = drift_slip_large(slip53);
+    if (FAST)
+        p.zeta = fma(L, dzeta, p.zeta);
+    else
+        p.zeta += L * dzeta;
     add_s<S_LIVE>(p, L);
 }
 

@@ -1,0 +1,33 @@
+"""The integer-pipe parts of the element maps (csrc/intpath.cuh), on the CPU:
+every value they decide has the bits of the FP64 sequence they stand for."""
+
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "sixtracklib_gb300", "csrc")
+
+
+@pytest.fixture(scope="module")
+def check(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("intpath") / "check")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-x", "c++", "-I" + CSRC,
+                    os.path.join(HERE, "intpath_check.cpp"), "-o", exe], check=True)
+
+    def run(what, n, seed):
+        out = subprocess.run([exe, what, str(n), str(seed)], check=True, capture_output=True,
+                             text=True).stdout
+        return [int(v) for v in out.split()]
+
+    return run
+
+
+@pytest.mark.parametrize("what", ["ordinary", "wide", "ties", "special"])
+def test_drift_slip_has_the_fp64_bits(check, what):
+    """Both policies' rvv - (1 + (xp^2 + yp^2) / 2)."""
+    n, undecided, different = check(what, 2_000_000, 7)
+    print(f"{what}: {undecided} of {n} left to the FP64 sequence")
+    assert different == 0
+    assert undecided < n
