@@ -728,10 +728,10 @@ __device__ __forceinline__ void reverse_elem(RState &s, Lam &l, const uint64_t *
         break;
     }
     case OP_MULTIPOLE:  // be_multipole/track.h:38-112
-        reverse_multipole<false>(s, l, rec + 1, (int)aux, a, e, on);
+        reverse_multipole<false>(s, l, rec + 1, (int)(aux & MP_ORDER), a, e, on);
         break;
     case OP_MULTIPOLE_CURV:
-        reverse_multipole<true>(s, l, rec + 1, (int)aux, a, e, on);
+        reverse_multipole<true>(s, l, rec + 1, (int)(aux & MP_ORDER), a, e, on);
         break;
     case OP_CAVITY: {  // be_cavity/track.h:39-67 + particles.h:5255-5297
         double gV = 0.0;

@@ -747,7 +747,7 @@ st_track_status_t st_DeviceLattice_set_parameters(st_DeviceLattice *L, int64_t n
         uint64_t const off = (uint64_t)ds.cs.elem_offset[(size_t)e];
         uint64_t const hdr = ds.cs.words[off];
         uint32_t const op = (uint32_t)(hdr & 0xFF);
-        uint32_t const order = (uint32_t)(hdr >> 32);
+        uint32_t const order = (uint32_t)(hdr >> 32) & MP_ORDER;
         if (kind[j] >= 0) {
             const uint64_t *bal = img.deref((uint64_t)e, 4);
             if ((op != OP_MULTIPOLE && op != OP_MULTIPOLE_CURV) || !bal ||
@@ -777,6 +777,14 @@ st_track_status_t st_DeviceLattice_set_parameters(st_DeviceLattice *L, int64_t n
         std::memcpy(&bits, &value[j], 8);
         ds.cs.words[where[(size_t)j].first] = bits;
         L->image[where[(size_t)j].second] = bits;
+    }
+    for (int64_t j = 0; j < num; ++j) {  // what the headers say of the coefficients
+        if (kind[j] < 0) continue;
+        uint64_t const off = (uint64_t)ds.cs.elem_offset[(size_t)element[j]];
+        uint64_t &hdr = ds.cs.words[off];
+        uint32_t const order = (uint32_t)(hdr >> 32) & MP_ORDER;
+        hdr = (hdr & 0xFFFFFFFFull) |
+              ((uint64_t)multipole_aux(&ds.cs.words[off + 1], order) << 32);
     }
     if (!cuda_ok(cudaMemcpy(ds.d, ds.cs.words.data(), ds.cs.words.size() * 8,
                             cudaMemcpyHostToDevice),

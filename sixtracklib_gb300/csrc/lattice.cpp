@@ -97,7 +97,7 @@ bool compile_lattice(const ImageView &img, uint64_t begin, uint64_t end,
             double const hxl = w2d(w[2]), hyl = w2d(w[3]);
             bool const curv = (hxl > 0.0) || (hyl > 0.0) || (hxl < 0.0) || (hyl < 0.0);
             op = curv ? OP_MULTIPOLE_CURV : OP_MULTIPOLE;
-            aux = (uint32_t)order;
+            aux = multipole_aux(bal, (uint32_t)order);
             p.assign(bal, bal + 2 * order + 2);
             if (curv) {
                 double const length = w2d(w[1]);

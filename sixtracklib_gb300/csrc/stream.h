@@ -17,8 +17,9 @@ enum Op : uint32_t {
     OP_END = 0,             // end of chunk
     OP_DRIFT = 1,           // [L]            aux bit0: global aperture check
     OP_DRIFT_EXACT = 2,     // [L]            aux bit0: global aperture check
-    OP_MULTIPOLE = 3,       // [bal 0..2n+1]  aux = order n
-    OP_MULTIPOLE_CURV = 4,  // [bal..., hxl, hyl, length, hxl/length, hyl/length]  aux = order n
+    OP_MULTIPOLE = 3,       // [bal 0..2n+1]  aux = order n | MP_ flags
+    OP_MULTIPOLE_CURV = 4,  // [bal..., hxl, hyl, length, hxl/length, hyl/length]
+                            // aux = order n | MP_ flags
     OP_CAVITY = 5,          // [voltage, k*frequency, deg2rad*lag]
     OP_XYSHIFT = 6,         // [-dx, -dy]
     OP_SROTATION = 7,       // [cos_z, sin_z]
@@ -72,6 +73,12 @@ enum Op : uint32_t {
 };
 
 constexpr uint32_t DRIFT_APERTURE = 1u;
+// Multipole aux word: the order and what is known of the coefficients
+// (multipole_aux).
+constexpr uint32_t MP_ORDER = 0xFFu;
+constexpr uint32_t MP_SKEW0 = 1u << 8;   // every skew coefficient is +-0
+constexpr uint32_t MP_PLUS = 1u << 9;    // every skew coefficient is +0, no other is -0
+constexpr uint32_t MP_DIPOLE0 = 1u << 10;  // bal[0] and bal[1] are +0
 // TriCub aux flags: mirror the grid coordinate in x / y / z (mirror_* == 1).
 constexpr uint32_t TRICUB_MIRROR_X = 1u;
 constexpr uint32_t TRICUB_MIRROR_Y = 2u;
@@ -94,6 +101,22 @@ constexpr uint32_t BB6D_SLICES = BB6D_ROUND - 1u;
 inline uint64_t make_header(uint32_t op, uint32_t nwords, uint32_t aux)
 {
     return (uint64_t)op | ((uint64_t)(nwords & 0xFFFFFFu) << 8) | ((uint64_t)aux << 32);
+}
+
+// The aux word of a multipole of order n with coefficients bal[0..2n+1]; made
+// again wherever a coefficient is changed.
+inline uint32_t multipole_aux(const uint64_t *bal, uint32_t order)
+{
+    constexpr uint64_t kMinusZero = (uint64_t)1 << 63;
+    uint64_t skew = 0;
+    bool minus_zero = false;
+    for (uint32_t k = 0; k <= order; ++k) {
+        skew |= bal[2 * k + 1];
+        minus_zero = minus_zero || bal[2 * k] == kMinusZero;
+    }
+    return order | ((skew << 1) == 0 ? MP_SKEW0 : 0u) |
+           (skew == 0 && !minus_zero ? MP_PLUS : 0u) |
+           ((bal[0] | bal[1]) == 0 ? MP_DIPOLE0 : 0u);
 }
 
 // Global aperture compare: |x| < limit  <=>  bits(|x|) < bits(limit) for a

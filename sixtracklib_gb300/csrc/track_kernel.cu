@@ -198,7 +198,7 @@ __device__ __forceinline__ int apply(PState &p, const uint64_t *rec, uint64_t hd
         if (aux & DRIFT_APERTURE) p.state &= (int64_t)inside_global(p, prm.xlim_bits, prm.ylim_bits);
         return 0;
     case OP_MULTIPOLE:
-        multipole<FAST, false>(p, rec, (int)aux);
+        multipole<FAST, false>(p, rec, aux);
         return 0;
     case OP_SROTATION:
         srotation<FAST>(p, rec);
@@ -214,7 +214,7 @@ __device__ __forceinline__ int apply(PState &p, const uint64_t *rec, uint64_t hd
         cavity(p, rec);
         return 0;
     case OP_MULTIPOLE_CURV:
-        multipole<FAST, true>(p, rec, (int)aux);
+        multipole<FAST, true>(p, rec, aux);
         return 0;
     case OP_DRIFT_EXACT:
         drift_exact<S_LIVE>(p, W(rec[1]));

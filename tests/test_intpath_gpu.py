@@ -58,3 +58,31 @@ def test_drift_at_the_edges(oracles, mode, p0c):
     for length in (1.0, 2.5, 1e-3, 0.0):
         e.Drift(length=length)
     _same(e, p.block, oracles[mode], mode)
+
+
+@pytest.mark.parametrize("mode", ["exact", "fast"])
+@pytest.mark.parametrize("chi", [1.0, 0.5])
+@pytest.mark.parametrize("order", [0, 1, 2, 3, 5])
+def test_multipole_zero_coefficients(oracles, mode, chi, order):
+    """Zero, minus-zero and nonzero coefficients at every order, coordinates
+    that are zeros of both signs, subnormal, huge, inf and NaN: signs of
+    zeros included."""
+    rng = np.random.default_rng(order)
+    v = np.array([0.0, -0.0, 1e-310, 1e-3, -2e-3, 0.7, 1e200, np.inf, np.nan])
+    x, y = (a.ravel() for a in np.meshgrid(v, v))
+    x, y = np.tile(x, 4), np.tile(y, 4)
+    p = lattices.gaussian_particles(x.size, seed=5)
+    p.x[:], p.y[:] = x, y
+    p.px[:81], p.py[81:162], p.px[162:243] = 0.0, -0.0, -0.0
+    p.py[162:243] = 0.0
+    p.chi[:] = chi
+    for trial in range(8):
+        bal = rng.normal(size=2 * order + 2) * 10.0 ** rng.uniform(-3, 0, 2 * order + 2)
+        bal[rng.random(bal.size) < 0.5] = 0.0
+        if trial < 6:
+            bal[1::2] = 0.0  # no skew component
+        if trial % 3 == 1:
+            bal[bal == 0.0] *= rng.choice([1.0, -1.0], (bal == 0.0).sum())
+        e = Elements()
+        e.Multipole(order=order, bal=bal)
+        _same(e, p.block, oracles[mode], mode)
