@@ -180,67 +180,70 @@ __device__ __forceinline__ int64_t ebe_index(const EbeDevConfig &c, int64_t pid,
     return out;
 }
 
-// Apply one element; returns 0 or -1 (reference status).  `lost` is set when
-// the particle leaves the aperture (state becomes 0).  The PLAIN
-// instantiation compiles only the maps of kPlainOps; the host chooses it
-// for lattices without any other opcode, so its fall-through (failure,
-// particle lost, as for an unknown type id) is never taken.
+// What became of a particle in an element.
+enum Passed : int { PASSED = 0, LOST = 1, FAILED = -1 };
+
+// Apply one element.  FAILED is the reference's status -1; p.state is left
+// as the reference's map leaves it.  The PLAIN instantiation compiles only
+// the maps of kPlainOps; the host chooses it for lattices without any other
+// opcode, so its fall-through (failure, particle lost, as for an unknown
+// type id) is never taken.  Maps that cannot lose a particle return a
+// constant, so the walk tests nothing after them.
 template <bool FAST, bool PLAIN, bool S_LIVE>
-__device__ __forceinline__ int apply(PState &p, const uint64_t *rec, uint64_t hdr,
-                                     const TrackParams &prm, int64_t cur_elem, int64_t cur_turn,
-                                     int64_t ord)
+__device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t hdr,
+                                        const TrackParams &prm, int64_t start_elem, int64_t ord)
 {
     uint32_t const op = (uint32_t)(hdr & 0xFF);
     uint32_t const aux = (uint32_t)(hdr >> 32);
+    auto limit = [&](bool inside) {
+        if (inside) return PASSED;
+        p.state = 0;
+        return LOST;
+    };
     switch (op) {
     case OP_DRIFT:
         drift<FAST, S_LIVE>(p, W(rec[1]));
-        if (aux & DRIFT_APERTURE) p.state &= (int64_t)inside_global(p, prm.xlim_bits, prm.ylim_bits);
-        return 0;
+        return limit(!(aux & DRIFT_APERTURE) || inside_global(p, prm.xlim_bits, prm.ylim_bits));
     case OP_MULTIPOLE:
         multipole<FAST, false>(p, rec, aux);
-        return 0;
+        return PASSED;
     case OP_SROTATION:
         srotation<FAST>(p, rec);
-        return 0;
+        return PASSED;
     case OP_XYSHIFT:
         p.x += W(rec[1]);
         p.y += W(rec[2]);
-        return 0;
+        return PASSED;
     case OP_LIMIT_ELLIPSE:
-        p.state &= (int64_t)inside_ellipse<FAST>(p, rec, aux);
-        return 0;
+        return limit(inside_ellipse<FAST>(p, rec, aux));
     case OP_CAVITY:
         cavity(p, rec);
-        return 0;
+        return PASSED;
     case OP_MULTIPOLE_CURV:
         multipole<FAST, true>(p, rec, aux);
-        return 0;
+        return PASSED;
     case OP_DRIFT_EXACT:
         drift_exact<S_LIVE>(p, W(rec[1]));
-        if (aux & DRIFT_APERTURE) p.state &= (int64_t)inside_global(p, prm.xlim_bits, prm.ylim_bits);
-        return 0;
+        return limit(!(aux & DRIFT_APERTURE) || inside_global(p, prm.xlim_bits, prm.ylim_bits));
     case OP_LIMIT_RECT:
-        p.state &= (int64_t)inside_rect(p, rec);
-        return 0;
+        return limit(inside_rect(p, rec));
     case OP_LIMIT_RECT_ELLIPSE:
-        p.state &= (int64_t)inside_rect_ellipse(p, rec);
-        return 0;
+        return limit(inside_rect_ellipse(p, rec));
     case OP_DIPEDGE:
         p.px += W(rec[1]) * p.x;
         p.py += W(rec[2]) * p.y;
-        return 0;
+        return PASSED;
     case OP_RF_MULTIPOLE:
         if constexpr (PLAIN) break;
         else {
             p = rf_multipole(p, rec, (int)aux);
-            return 0;
+            return PASSED;
         }
     case OP_BB4D:
         if constexpr (PLAIN) break;
         else {
             p = beam_beam_4d(p, rec);
-            return 0;
+            return PASSED;
         }
     case OP_BB6D:
         if constexpr (PLAIN) break;
@@ -249,94 +252,102 @@ __device__ __forceinline__ int apply(PState &p, const uint64_t *rec, uint64_t hd
                 p = beam_beam_6d<true, FAST>(p, rec, (int)(aux & BB6D_SLICES));
             else
                 p = beam_beam_6d<false, FAST>(p, rec, (int)aux);
-            return 0;
+            return PASSED;
         }
     case OP_SC_COASTING:
         if constexpr (PLAIN) break;
         else {
             p = sc_coasting(p, rec);
-            return 0;
+            return PASSED;
         }
     case OP_SC_QGAUSS:
         if constexpr (PLAIN) break;
         else {
             p = sc_qgauss<FAST>(p, rec, aux);
-            return 0;
+            return PASSED;
         }
     case OP_SC_INTERP:
         if constexpr (PLAIN) break;
         else {
             p = sc_interpolated(p, rec, aux);
-            return 0;
+            return PASSED;
         }
     case OP_TRICUB:
         if constexpr (PLAIN) break;
         else {
             p = tricub<FAST>(p, rec, aux);
-            return p.state == 1 ? 0 : -1;  // outside the grid: lost, failure
+            return p.state == 1 ? PASSED : FAILED;  // outside the grid: lost, failure
         }
     case OP_MONITOR: {
         uint64_t *out = reinterpret_cast<uint64_t *>(rec[8]);
-        if (out == nullptr) return 0;
+        if (out == nullptr) return PASSED;
         int64_t const j = monitor_index(rec, p.at_turn, p.pid);
-        if (j < 0) return 0;
+        if (j < 0) return PASSED;
         if (j >= (int64_t)rec[9]) {
             p.state = 0;
-            return -1;
+            return FAILED;
         }
-        store_record(p, out, (int64_t)rec[9], j, cur_elem, cur_turn,
+        store_record(p, out, (int64_t)rec[9], j, start_elem + ord, p.at_turn,
                      p.lazy_s ? prm.s_table[ord] : p.s);
-        return 0;
+        return PASSED;
     }
     case OP_NOP:
-        return 0;
+        return PASSED;
     case OP_FAIL:
-        return -1;
+        return FAILED;
     default:  // OP_FAIL_LOST: unknown type id
         break;
     }
     p.state = 0;
-    return -1;
+    return FAILED;
 }
 
 }  // namespace
 
 // The records of one staged chunk, in order, for the calling thread's
-// particle (lanes whose particle takes no part are predicated off).
+// particle.  Only lanes that take part walk; one whose particle stops leaves
+// the loop, so nothing has to reconverge per element.  The next record's
+// header is read before the element is applied: with one or two warps per
+// scheduler (10,000 particles) the walk's time is its chain of latencies,
+// and the header's shared-memory read was a link of it.
 // S_LIVE (block-uniform for the pass): some particle of the block
-// accumulates s, so drifts carry the s update.
-template <bool FAST, bool PLAIN, bool S_LIVE>
+// accumulates s, so drifts carry the s update.  EBE: element-by-element
+// output, whose particles may enter an element already lost (the reference
+// checks the state after the map).
+template <bool FAST, bool PLAIN, bool S_LIVE, bool EBE>
 __device__ __forceinline__ void walk_chunk(PState &p, const uint64_t *rec, const TrackParams &prm,
                                            bool &part, bool &active, int &status,
-                                           int64_t &stop_elem, int64_t &ord, int64_t &ae,
-                                           int64_t start_elem)
+                                           int64_t &stop_elem, int64_t &ord, int64_t start_elem)
 {
-    while (true) {
-        uint64_t const hdr = rec[0];
-        uint32_t const nw = (uint32_t)((hdr >> 8) & 0xFFFFFF);
-        if ((uint32_t)(hdr & 0xFF) == OP_END || nw == 0) break;
-        if (part) {
-            if (prm.mode == MODE_EBE) {
-                int64_t const j = ebe_index(prm.ebe, p.pid, ae, p.at_turn);
-                if (j >= 0 && j < prm.ebe_cap)
-                    store_record(p, prm.ebe_out, prm.ebe_cap, j, ae, p.at_turn,
-                                 p.lazy_s ? prm.s_table[ord] : p.s);
-            }
-            int const rc =
-                apply<FAST, PLAIN, S_LIVE>(p, rec, hdr, prm, start_elem + ord, p.at_turn, ord);
-            if (rc != 0 || p.state != 1) {
-                status |= rc;
-                part = false;
-                active = false;
-                stop_elem = ord;
-                if (p.lazy_s) p.s = prm.s_table[ord + 1];
-            } else {
-                ++ae;
-            }
+    if (!part) return;
+    int64_t const first = ord;
+    uint64_t hdr = rec[0];
+    uint32_t o = 0;
+    // a chunk ends with an OP_END record (or zero padding, which reads as one)
+    while ((uint32_t)(hdr & 0xFF) != OP_END) {
+        const uint64_t *const next = rec + ((hdr >> 8) & 0xFFFFFFu);
+        uint64_t const next_hdr = next[0];
+        if constexpr (EBE) {
+            int64_t const ae = start_elem + first + o;
+            int64_t const j = ebe_index(prm.ebe, p.pid, ae, p.at_turn);
+            if (j >= 0 && j < prm.ebe_cap)
+                store_record(p, prm.ebe_out, prm.ebe_cap, j, ae, p.at_turn,
+                             p.lazy_s ? prm.s_table[first + o] : p.s);
         }
-        ++ord;
-        rec += nw;
+        Passed const rc = apply<FAST, PLAIN, S_LIVE>(p, rec, hdr, prm, start_elem, first + o);
+        if (rc != PASSED || (EBE && p.state != 1)) {
+            if (rc == FAILED) status |= -1;
+            part = false;
+            active = false;
+            stop_elem = first + o;
+            if (p.lazy_s) p.s = prm.s_table[first + o + 1];
+            return;
+        }
+        ++o;
+        rec = next;
+        hdr = next_hdr;
     }
+    ord = first + o;
 }
 
 __device__ __forceinline__ void mbar_inval(uint64_t *bar)
@@ -432,7 +443,6 @@ __device__ __forceinline__ void track_block(const TrackParams &prm, int64_t t, u
         // some particle of the block accumulates s in this pass (block-uniform)
         bool const s_live = __syncthreads_or(part && !p.lazy_s);
         int64_t ord = 0;  // element ordinal within the turn / line
-        int64_t ae = start_elem;
         for (int c = 0; c < nch; ++c) {
             int buf = c;
             if (!resident) {
@@ -446,12 +456,15 @@ __device__ __forceinline__ void track_block(const TrackParams &prm, int64_t t, u
                 }
             }
             const uint64_t *rec = bufs + (size_t)buf * cw;
-            if (s_live)
-                walk_chunk<FAST, PLAIN, true>(p, rec, prm, part, active, status, stop_elem, ord,
-                                              ae, start_elem);
+            if (prm.mode == MODE_EBE)
+                walk_chunk<FAST, PLAIN, true, true>(p, rec, prm, part, active, status, stop_elem,
+                                                    ord, start_elem);
+            else if (s_live)
+                walk_chunk<FAST, PLAIN, true, false>(p, rec, prm, part, active, status, stop_elem,
+                                                     ord, start_elem);
             else
-                walk_chunk<FAST, PLAIN, false>(p, rec, prm, part, active, status, stop_elem, ord,
-                                               ae, start_elem);
+                walk_chunk<FAST, PLAIN, false, false>(p, rec, prm, part, active, status,
+                                                      stop_elem, ord, start_elem);
             if (!resident) {
                 __syncthreads();  // every warp is done with this stage buffer
                 if (threadIdx.x == 0) {
