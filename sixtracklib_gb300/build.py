@@ -3,7 +3,7 @@
 ``build()`` compiles the host C++ (CObjects buffer, lattice compiler) with
 g++ and the CUDA sources for sm_103a with nvcc, in parallel, and links
 ``sixtracklib_gb300/lib/libsixtracklib_gb300.so`` in the source tree.  The
-tracking kernel's translation unit is compiled with ``-fmad=false``: the
+tracking kernel's translation units are compiled with ``-fmad=false``: the
 exact arithmetic policy relies on it, the fast one uses explicit fma().
 """
 
@@ -25,6 +25,8 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 HOST_SOURCES = ["buffer.cpp", "lattice.cpp", "output_buffer.cpp", "aliases.cpp"]
 CUDA_SOURCES = {
     "track_kernel.cu": ["-fmad=false"],
+    "track_kernel_plain.cu": ["-fmad=false"],
+    "track_kernel_full.cu": ["-fmad=false"],
     "engine.cu": [],
     "probe.cu": [],
     "compact.cu": [],

@@ -115,7 +115,7 @@ struct Plan {
     int32_t num_items = 0;
     unsigned grid = 0;
     size_t smem = 0;
-    bool plain = false;  // every variant is a plain ring: the plain-ring kernel
+    LatticeKind kind = KIND_FULL;  // covers every variant
     void release()
     {
         if (d_variants) cudaFree(d_variants);
@@ -178,10 +178,11 @@ bool build_plan(st_BatchTracker *b, const Shape &sh, const std::vector<uint64_t 
     Plan p;
     p.shape = sh;
     p.smem = track_smem_bytes(sh.stages, max_chunk_words(b));
-    p.plain = true;
-    for (const auto &v : b->views) p.plain = p.plain && plain_lattice(v.op_mask);
+    uint32_t ops = 0;
+    for (const auto &v : b->views) ops |= v.op_mask;
+    p.kind = lattice_kind(ops);
     int per_sm = 0;
-    int rc = batch_ctas_per_sm(b->fast, p.plain, sh.threads, sh.blocks_per_sm, p.smem, &per_sm);
+    int rc = batch_ctas_per_sm(b->fast, p.kind, sh.threads, sh.blocks_per_sm, p.smem, &per_sm);
     if (rc != 0 || per_sm <= 0) {
         set_error("batch: launch shape does not fit an SM (threads " +
                   std::to_string(sh.threads) + ", stages " + std::to_string(sh.stages) + ")");
@@ -272,7 +273,7 @@ bool enqueue_turns(st_BatchTracker *b, const Plan &p, int64_t turns, cudaStream_
         L.base_turn = b->d_base;
         L.turn_offset = std::min(turns, (k + 1) * tpl);
         L.fast = b->fast;
-        L.plain = p.plain;
+        L.kind = p.kind;
         L.threads = p.shape.threads;
         L.blocks_per_sm = p.shape.blocks_per_sm;
         L.grid = p.grid;

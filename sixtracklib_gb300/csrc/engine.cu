@@ -29,6 +29,7 @@
 #include "kernel_api.h"
 #include "device_guard.h"
 #include "lattice.h"
+#include "leadkick.cuh"
 
 extern "C" uint64_t stg_buffer_generation(const st_Buffer *b);
 
@@ -783,8 +784,14 @@ st_track_status_t st_DeviceLattice_set_parameters(st_DeviceLattice *L, int64_t n
         uint64_t const off = (uint64_t)ds.cs.elem_offset[(size_t)element[j]];
         uint64_t &hdr = ds.cs.words[off];
         uint32_t const order = (uint32_t)(hdr >> 32) & MP_ORDER;
-        hdr = (hdr & 0xFFFFFFFFull) |
-              ((uint64_t)multipole_aux(&ds.cs.words[off + 1], order) << 32);
+        uint32_t aux = multipole_aux(&ds.cs.words[off + 1], order);
+        // a record compiled with a lead block has room for another
+        uint64_t const at = 1 + 2 * (uint64_t)order + 2;
+        if ((hdr & 0xFF) == OP_MULTIPOLE &&
+            ((hdr >> 8) & 0xFFFFFF) == at + (uint64_t)lead_words((int)order) &&
+            lead_block(&ds.cs.words[off + 1], (int)order, &ds.cs.words[off + at]))
+            aux |= MP_LEAD;
+        hdr = (hdr & 0xFFFFFFFFull) | ((uint64_t)aux << 32);
     }
     if (!cuda_ok(cudaMemcpy(ds.d, ds.cs.words.data(), ds.cs.words.size() * 8,
                             cudaMemcpyHostToDevice),

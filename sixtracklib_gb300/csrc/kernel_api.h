@@ -14,7 +14,7 @@ enum TrackMode : int32_t { MODE_UNTIL = 0, MODE_LINE = 1, MODE_EBE = 2 };
 
 enum ErrorBits : int32_t { ERR_PIPELINE_TIMEOUT = 1 };
 
-// Opcodes of the plain-ring kernel instantiation: drifts, multipoles,
+// Opcodes of the plain-ring kernel instantiations: drifts, multipoles,
 // shifts, rotations, dipole edges, cavities, apertures and monitors.  A
 // lattice with none of the beam-field, space-charge or RF-multipole maps is
 // tracked by a kernel compiled without them, which needs fewer registers
@@ -26,7 +26,17 @@ constexpr uint32_t kPlainOps =
     (1u << OP_DIPEDGE) | (1u << OP_MONITOR) | (1u << OP_NOP) | (1u << OP_FAIL) |
     (1u << OP_FAIL_LOST);
 
-inline bool plain_lattice(uint32_t op_mask) { return (op_mask & ~kPlainOps) == 0u; }
+// The kernel is compiled for three kinds of lattices: plain rings without
+// and with lead blocks (the kick of leadkick.cuh compiled in costs a ring of
+// quadrupoles 3.5 %: 10,000 protons x 100 turns of the FODO ring 9.9 against
+// 10.3 ms), and any lattice.
+enum LatticeKind : int { KIND_SIMPLE = 0, KIND_PLAIN = 1, KIND_FULL = 2 };
+
+inline LatticeKind lattice_kind(uint32_t op_mask)
+{
+    if (op_mask & ~(kPlainOps | OPM_LEAD)) return KIND_FULL;
+    return (op_mask & OPM_LEAD) ? KIND_PLAIN : KIND_SIMPLE;
+}
 
 struct EbeDevConfig {
     int64_t order;
@@ -65,8 +75,7 @@ struct TrackParams {
 // error code of the launch (0 on success).
 // blocks_per_sm selects the register tier: 1 (up to 255 registers, no
 // spills) or 2 (at most 128 registers per thread, two CTAs per SM).
-// prm.op_mask selects the instantiation: the plain-ring kernel when every
-// opcode present is in kPlainOps, the full kernel otherwise.
+// prm.op_mask selects the instantiation (lattice_kind).
 int launch_track(const TrackParams &prm, bool fast, int threads, int blocks_per_sm,
                  void *stream);
 size_t track_smem_bytes(int stages, int chunk_words);
@@ -98,7 +107,7 @@ struct BatchLaunch {
     const int64_t *base_turn;     // device: until_turn = *base_turn + turn_offset
     int64_t turn_offset;
     bool fast;
-    bool plain;                   // every variant is a plain ring (kPlainOps)
+    LatticeKind kind;             // covers every variant
     int threads, blocks_per_sm;
     unsigned grid;
     size_t smem;
@@ -106,7 +115,7 @@ struct BatchLaunch {
 
 // Set the kernel's shared-memory limit to `smem` and report how many CTAs
 // of `threads` fit on one SM.  Returns the CUDA error code.
-int batch_ctas_per_sm(bool fast, bool plain, int threads, int blocks_per_sm, size_t smem,
+int batch_ctas_per_sm(bool fast, LatticeKind kind, int threads, int blocks_per_sm, size_t smem,
                       int *per_sm);
 int launch_batch(const BatchLaunch &b, void *stream);
 

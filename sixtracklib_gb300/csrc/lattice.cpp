@@ -9,6 +9,8 @@
 // contiguously after the fixed part.
 #include "lattice.h"
 
+#include "leadkick.cuh"
+
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -108,6 +110,13 @@ bool compile_lattice(const ImageView &img, uint64_t begin, uint64_t end,
                 // derivative kernels' form of the b1 / a1 terms
                 p.push_back(d2w(length > 0.0 ? hxl / length : 0.0));
                 p.push_back(d2w(length > 0.0 ? hyl / length : 0.0));
+            } else {
+                uint64_t blk[64];
+                if (lead_block(bal, (int)order, blk)) {
+                    aux |= MP_LEAD;
+                    op_mask |= OPM_LEAD;
+                    p.insert(p.end(), blk, blk + lead_words((int)order));
+                }
             }
             break;
         }

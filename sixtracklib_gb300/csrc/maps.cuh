@@ -16,6 +16,7 @@
 
 #include "exp_table.h"
 #include "intpath.cuh"
+#include "leadkick.cuh"
 #include "stream.h"
 
 namespace stg {
@@ -287,11 +288,61 @@ __device__ __forceinline__ double plus_zero(double v)
     return __hiloint2double((int)(((hi << 1) | lo) ? hi : 0u), (int)lo);
 }
 
-template <bool FAST, bool CURV>
+// v - a and fma(-chi, a, v), out of line (see chi_kick)
+static __device__ __noinline__ double less(double v, double a) { return v - a; }
+static __device__ __noinline__ double less_product(double v, double chi, double a)
+{
+    return fma(-chi, a, v);
+}
+
+__device__ __forceinline__ bool same_bits(double a, double b)
+{
+    return __double2hiint(a) == __double2hiint(b) && __double2loint(a) == __double2loint(b);
+}
+
+// The kick of a multipole with a lead block (leadkick.cuh); false where a
+// rounding is left open, with p unchanged.  u_1 x and u_1 y with the small
+// corrections are formed at both ends of their bounds; where these differ
+// the momenta still decide, being rounded more coarsely.  All lanes of the
+// warp in range or none (the others would run both sequences).
+template <bool FAST>
+__device__ __forceinline__ bool lead_kick(PState &p, const uint64_t *bal, int order)
+{
+    double const x = p.x, y = p.y, chi = p.chi;
+    if (!__all_sync(__activemask(), lead_in_range(x, y, bal + 2 * order + 2) &&
+                                        (FAST || is_one(chi))))
+        return false;
+    if (FAST) {
+        double c1, w[2];
+        if (!lead_fast(x, y, bal, order, &c1, w)) return false;
+        double const a = fma(x, c1, -w[0]), b = fma(x, c1, -w[1]);
+        double const dpy = y * c1;
+        double const px = fma(-chi, a, p.px);
+        if (!same_bits(a, b) && !same_bits(px, less_product(p.px, chi, b))) return false;
+        p.px = px;
+        p.py = fma(chi, dpy, p.py);
+    } else {
+        double u1, e1[2], e2[2];
+        if (!lead_exact(x, y, bal, order, &u1, e1, e2)) return false;
+        double const kx = u1 * x, ky = u1 * y;
+        double const a = plus_zero(kx - e1[0]), b = plus_zero(kx - e1[1]);
+        double const c = plus_zero(ky + e2[0]), d = plus_zero(ky + e2[1]);
+        double const px = p.px - a, py = p.py + c;
+        if (!same_bits(a, b) && !same_bits(px, less(p.px, b))) return false;
+        if (!same_bits(c, d) && !same_bits(py, less(p.py, -d))) return false;
+        p.px = px;
+        p.py = py;
+    }
+    return true;
+}
+
+template <bool FAST, bool CURV, bool LEAD>
 __device__ __forceinline__ void multipole(PState &p, const uint64_t *rec, uint32_t aux)
 {
     const uint64_t *bal = rec + 1;
     int const order = (int)(aux & MP_ORDER);
+    if (LEAD && !CURV && (aux & MP_LEAD) && (!FAST || order >= 3))
+        if (lead_kick<FAST>(p, bal, order)) return;
     double dpx = W(bal[2 * order]);
     double dpy = W(bal[2 * order + 1]);
     double const x = p.x, y = p.y, chi = p.chi;

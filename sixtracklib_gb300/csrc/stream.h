@@ -17,7 +17,8 @@ enum Op : uint32_t {
     OP_END = 0,             // end of chunk
     OP_DRIFT = 1,           // [L]            aux bit0: global aperture check
     OP_DRIFT_EXACT = 2,     // [L]            aux bit0: global aperture check
-    OP_MULTIPOLE = 3,       // [bal 0..2n+1]  aux = order n | MP_ flags
+    OP_MULTIPOLE = 3,       // [bal 0..2n+1]  aux = order n | MP_ flags; with
+                            // MP_LEAD the lead block follows (leadkick.cuh)
     OP_MULTIPOLE_CURV = 4,  // [bal..., hxl, hyl, length, hxl/length, hyl/length]
                             // aux = order n | MP_ flags
     OP_CAVITY = 5,          // [voltage, k*frequency, deg2rad*lag]
@@ -72,6 +73,10 @@ enum Op : uint32_t {
     OP_COUNT
 };
 
+// Beside the opcodes in a lattice's op mask: some multipole has a lead block.
+constexpr uint32_t OPM_LEAD = 1u << 31;
+static_assert(OP_COUNT <= 31, "op mask bits");
+
 constexpr uint32_t DRIFT_APERTURE = 1u;
 // Multipole aux word: the order and what is known of the coefficients
 // (multipole_aux).
@@ -79,6 +84,7 @@ constexpr uint32_t MP_ORDER = 0xFFu;
 constexpr uint32_t MP_SKEW0 = 1u << 8;   // every skew coefficient is +-0
 constexpr uint32_t MP_PLUS = 1u << 9;    // every skew coefficient is +0, no other is -0
 constexpr uint32_t MP_DIPOLE0 = 1u << 10;  // bal[0] and bal[1] are +0
+constexpr uint32_t MP_LEAD = 1u << 11;     // the quadrupole term leads
 // TriCub aux flags: mirror the grid coordinate in x / y / z (mirror_* == 1).
 constexpr uint32_t TRICUB_MIRROR_X = 1u;
 constexpr uint32_t TRICUB_MIRROR_Y = 2u;
@@ -136,7 +142,7 @@ struct StreamInfo {
     int32_t chunk_words = 0;
     int32_t max_record_words = 0;
     int32_t num_monitors = 0;
-    uint32_t op_mask = 0;  // bit per opcode present
+    uint32_t op_mask = 0;  // bit per opcode present, OPM_LEAD
 };
 
 }  // namespace stg

@@ -1,5 +1,6 @@
-"""The integer-pipe parts of the element maps (csrc/intpath.cuh), on the CPU:
-every value they decide has the bits of the FP64 sequence they stand for."""
+"""The integer- and FP32-pipe parts of the element maps (csrc/intpath.cuh,
+csrc/leadkick.cuh), on the CPU: every value they decide has the bits of the
+FP64 sequence they stand for."""
 
 import os
 import subprocess
@@ -28,6 +29,16 @@ def check(tmp_path_factory):
 def test_drift_slip_has_the_fp64_bits(check, what):
     """Both policies' rvv - (1 + (xp^2 + yp^2) / 2)."""
     n, undecided, different = check(what, 2_000_000, 7)
+    print(f"{what}: {undecided} of {n} left to the FP64 sequence")
+    assert different == 0
+    assert undecided < n
+
+
+@pytest.mark.parametrize("what", ["lead exact", "lead fast", "lead exact wide", "lead fast wide"])
+def test_lead_kick_has_the_fp64_bits(check, what):
+    """Both policies' kicks of quadrupoles with multipole errors, at 1 mm with
+    small errors and at 5 mm with errors 100 times larger."""
+    n, undecided, different = check(what, 400_000, 11)
     print(f"{what}: {undecided} of {n} left to the FP64 sequence")
     assert different == 0
     assert undecided < n

@@ -1,4 +1,5 @@
-"""The integer-pipe parts of the element maps (csrc/intpath.cuh) on the GPU,
+"""The integer- and FP32-pipe parts of the element maps (csrc/intpath.cuh,
+csrc/leadkick.cuh) on the GPU,
 bit for bit against the oracle (exact policy) and its restatement of the
 fast policy, at the edges of the ranges they decide."""
 
@@ -86,3 +87,55 @@ def test_multipole_zero_coefficients(oracles, mode, chi, order):
         e = Elements()
         e.Multipole(order=order, bal=bal)
         _same(e, p.block, oracles[mode], mode)
+
+
+@pytest.mark.parametrize("mode", ["exact", "fast"])
+@pytest.mark.parametrize("order", [2, 3, 4, 5, 10])
+@pytest.mark.parametrize("size", [1e-6, 1e-3, 8e-3, 40e-3])
+def test_lead_kick(oracles, mode, order, size):
+    """Quadrupoles with multipole errors (lead blocks) of either sign, at
+    amplitudes inside, across and beyond their range, on and near the axes;
+    one drift between them so that momenta act."""
+    rng = np.random.default_rng(order)
+    n = 2000
+    p = lattices.gaussian_particles(n, seed=order, sx=size, sy=size)
+    p.x[:40], p.y[40:80] = 0.0, -0.0
+    p.x[80:160] *= 1e-9
+    p.y[160:240] *= 10.0 ** rng.uniform(-30, 0, 80)
+    p.x[240:260], p.y[240:260] = 0.0, 0.0
+    p.px[260:400] = 0.0
+    p.chi[1000:1032] = 0.5
+    e = Elements()
+    for trial in range(24):
+        knl = np.zeros(order + 1)
+        knl[1] = rng.choice([-1, 1]) * rng.uniform(0.01, 0.05)
+        for k in range(2, order + 1):
+            knl[k] = rng.normal(0.0, 10.0 ** rng.uniform(-6, -2) * 10.0 ** -k)
+        e.Multipole(knl=list(knl))
+        e.Drift(length=float(rng.uniform(0.1, 2.0)))
+    _same(e, p.block, oracles[mode], mode)
+
+
+def test_lead_block_follows_the_parameters(oracles):
+    """A parameter change that ends or restores the lead of the quadrupole
+    term takes effect (the header and the block are made again)."""
+    import torch
+
+    from sixtracklib_gb300.autodiff import DifferentiableLattice, apply_values
+
+    e = Elements()
+    for k1 in (0.03, -0.02):
+        e.Multipole(knl=[0.0, k1, 1e-6, 1e-7], ksl=[0.0, 0.0, 0.0, 0.0])
+        e.Drift(length=1.0)
+    params = [(0, "knl", 1), (0, "knl", 2), (2, "ksl", 3), (2, "knl", 0)]
+    lat = DifferentiableLattice(e, params, "mode=exact")
+    p = lattices.gaussian_particles(500, seed=4)
+    for values in ([0.03, 1e-6, 0.0, 0.0], [1e-7, 5.0, 0.0, 0.0], [-0.04, -3e-6, 2e-3, 0.0],
+                   [0.02, 2e-6, 0.0, 1e-5], [0.015, 1e-6, 0.0, 0.0]):
+        lat.set_values(torch.tensor(values, dtype=torch.float64))
+        exp = p.block.copy()
+        now = apply_values(e, params, values)
+        assert oracles["exact"].track_until(now.cbuffer.to_image(), exp, 1) == 0
+        cols = torch.from_numpy(p.block.copy().view(np.int64)).cuda()
+        assert lat.tracker.track_until(cols, 1) == 0
+        assert np.array_equal(cols.cpu().numpy().view(np.uint64), exp)
