@@ -611,12 +611,75 @@ __device__ __noinline__ RevState reverse_bb6d(RevState r, const uint64_t *rec, i
     return r;
 }
 
+// The parameter list's entries of one multipole: d(dpx, dpy)/d bal[2k] =
+// chi (-Re z^k, Im z^k), / d bal[2k+1] = chi (Im z^k, Re z^k), with cx, cy =
+// chi times lambda_px, lambda_py (hxl_l, hyl_l: the curvature ratios or 0).
+template <bool CURV>
+__device__ __forceinline__ void multipole_grad(double x, double y, double cx, double cy,
+                                               double hxl_l, double hyl_l, const AdjParams &a,
+                                               int32_t j0, int32_t j1, bool on)
+{
+    for (int32_t j = j0; j < j1; ++j) {
+        int const k2 = a.pkind[j];
+        double g = 0.0;
+        if (on && k2 >= 0) {
+            int const kk = k2 >> 1;
+            double zr = 1.0, zi = 0.0;
+            if (kk > 0) {
+                zr = x;
+                zi = y;
+                for (int k = 1; k < kk; ++k) {
+                    double const t = fma(zr, x, -zi * y);
+                    zi = fma(zr, y, zi * x);
+                    zr = t;
+                }
+            }
+            g = (k2 & 1) ? fma(cx, zi, cy * zr) : fma(-cx, zr, cy * zi);
+            if (CURV && k2 == 0) g -= cx * x * hxl_l;
+            if (CURV && k2 == 1) g += cy * y * hyl_l;
+        }
+        add_grad(a, j, g, on);
+    }
+}
+
+// chi v, out of line for the particles with chi != 1 (a predicated-off FP64
+// instruction occupies the pipe)
+__device__ __noinline__ double times(double chi, double v) { return chi * v; }
+
+// A quadrupole (order 1, no skew or dipole term): the kick (-chi b x, chi b y)
+// taken back and its transposed Jacobian, 4 FP64 instructions instead of the
+// 12 of the general form.
+__device__ __forceinline__ void reverse_quadrupole(RState &s, Lam &l, double b1,
+                                                   const AdjParams &a, int32_t j0, int32_t j1,
+                                                   bool on)
+{
+    double const x = s.x, y = s.y, lpx = l.px, lpy = l.py;
+    bool const one = is_one(s.chi);
+    if (on) {
+        double b = b1;
+        if (!one) b = times(s.chi, b1);
+        s.px = fma(b, x, s.px);
+        s.py = fma(-b, y, s.py);
+        l.x = fma(-b, lpx, l.x);
+        l.y = fma(b, lpy, l.y);
+    }
+    if (j0 < j1) {  // warp-uniform
+        double cx = lpx, cy = lpy;
+        if (!one) {
+            cx = times(s.chi, lpx);
+            cy = times(s.chi, lpy);
+        }
+        multipole_grad<false>(x, y, cx, cy, 0.0, 0.0, a, j0, j1, on);
+    }
+}
+
 // Multipole (be_multipole/track.h:38-112), with the curvature terms only in
 // the CURV instantiation: a runtime branch around them is if-converted, and
 // predicated-off FP64 instructions still occupy the FP64 pipe.
 template <bool CURV>
 __device__ __forceinline__ void reverse_multipole(RState &s, Lam &l, const uint64_t *bal, int n,
-                                                  const AdjParams &a, int64_t e, bool on)
+                                                  const AdjParams &a, int32_t j0, int32_t j1,
+                                                  bool on)
 {
     double const chi = s.chi, x = s.x, y = s.y;
     // curvature words 2n+2.. : hxl, hyl, length, hxl / length, hyl / length
@@ -646,51 +709,28 @@ __device__ __forceinline__ void reverse_multipole(RState &s, Lam &l, const uint6
             l.d += lpx * hxl - lpy * hyl;
         }
     }
-    int32_t const j0 = a.pbeg ? a.pbeg[e] : 0, j1 = a.pbeg ? a.pbeg[e + 1] : 0;
-    if (j0 < j1) {  // warp-uniform
-        // d(dpx, dpy)/d bal[2k] = chi (-Re z^k, Im z^k); / d bal[2k+1] = chi (Im z^k, Re z^k)
-        double const cx = chi * lpx, cy = chi * lpy;
-        for (int32_t j = j0; j < j1; ++j) {
-            int const k2 = a.pkind[j];
-            double g = 0.0;
-            if (on && k2 >= 0) {
-                int const kk = k2 >> 1;
-                double zr = 1.0, zi = 0.0;
-                if (kk > 0) {
-                    zr = x;
-                    zi = y;
-                    for (int k = 1; k < kk; ++k) {
-                        double const t = fma(zr, x, -zi * y);
-                        zi = fma(zr, y, zi * x);
-                        zr = t;
-                    }
-                }
-                g = (k2 & 1) ? fma(cx, zi, cy * zr) : fma(-cx, zr, cy * zi);
-                if (CURV && k2 == 0) g -= cx * x * hxl_l;
-                if (CURV && k2 == 1) g += cy * y * hyl_l;
-            }
-            add_grad(a, j, g, on);
-        }
-    }
+    if (j0 < j1)  // warp-uniform
+        multipole_grad<CURV>(x, y, chi * lpx, chi * lpy, hxl_l, hyl_l, a, j0, j1, on);
 }
 
 // Restore the input of one element from its output (state s) and apply
 // lambda <- J^T lambda at that input.  `on` is false for lanes that do not
-// take part (they still join the warp reductions).  The 6D beam-beam
+// take part (they still join the warp reductions); `first` is the record's
+// first parameter, [j0, j1) its entries of the parameter list.  The 6D beam-beam
 // reverse is compiled in only where BB6D is set: its call site alone costs
 // lattices without the element a few percent (registers saved around it).
 template <bool BB6D>
-__device__ __forceinline__ void reverse_elem(RState &s, Lam &l, const uint64_t *rec,
-                                             const AdjParams &a, int64_t e, bool on)
+__device__ __forceinline__ void reverse_elem(RState &s, Lam &l, const uint64_t *rec, uint64_t hdr,
+                                             double first, const AdjParams &a, int32_t j0,
+                                             int32_t j1, bool on)
 {
-    uint64_t const hdr = rec[0];
     uint32_t const op = (uint32_t)(hdr & 0xFF);
     uint32_t const aux = (uint32_t)(hdr >> 32);
     switch (op) {
     case OP_DRIFT: {  // be_drift/track.h:45-67
         if (!on) break;
         // input from output: x -= L rpp px, zeta -= L (rvv - 1 - rpp^2 (px^2 + py^2) / 2)
-        double const L = W(rec[1]);
+        double const L = first;
         double const px = s.px, py = s.py;
         double const a_ = L * s.rpp;
         s.x = fma(-a_, px, s.x);
@@ -728,10 +768,13 @@ __device__ __forceinline__ void reverse_elem(RState &s, Lam &l, const uint64_t *
         break;
     }
     case OP_MULTIPOLE:  // be_multipole/track.h:38-112
-        reverse_multipole<false>(s, l, rec + 1, (int)(aux & MP_ORDER), a, e, on);
+        if ((aux & (MP_ORDER | MP_SKEW0 | MP_DIPOLE0)) == (1u | MP_SKEW0 | MP_DIPOLE0))
+            reverse_quadrupole(s, l, W(rec[3]), a, j0, j1, on);
+        else
+            reverse_multipole<false>(s, l, rec + 1, (int)(aux & MP_ORDER), a, j0, j1, on);
         break;
     case OP_MULTIPOLE_CURV:
-        reverse_multipole<true>(s, l, rec + 1, (int)(aux & MP_ORDER), a, e, on);
+        reverse_multipole<true>(s, l, rec + 1, (int)(aux & MP_ORDER), a, j0, j1, on);
         break;
     case OP_CAVITY: {  // be_cavity/track.h:39-67 + particles.h:5255-5297
         double gV = 0.0;
@@ -746,10 +789,7 @@ __device__ __forceinline__ void reverse_elem(RState &s, Lam &l, const uint64_t *
             refresh_lz(s, l);
             gV = lP * s.q * sph / s.energy0;
         }
-        if (a.pbeg) {
-            for (int32_t j = a.pbeg[e]; j < a.pbeg[e + 1]; ++j)
-                add_grad(a, j, a.pkind[j] < 0 ? gV : 0.0, on);
-        }
+        for (int32_t j = j0; j < j1; ++j) add_grad(a, j, a.pkind[j] < 0 ? gV : 0.0, on);
         break;
     }
     case OP_RF_MULTIPOLE:
@@ -872,8 +912,29 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm) adjoint_kernel(A
             long long const v = __shfl_xor_sync(0xFFFFFFFFu, wl, o);
             wl = v > wl ? v : wl;
         }
-        for (int64_t e = (int64_t)wl; e >= 0; --e)
-            reverse_elem<BB6D>(s, l, a.stream + a.elem_offset[e], a, e, act && e <= mine);
+        // The walk reads ahead: the offset of the record two elements on,
+        // the header, first parameter and parameter-list entry of the next.
+        // With one warp per scheduler (16,384 particles) an element's time
+        // was its chain of three dependent global reads plus its FP64
+        // instructions; with the short quadrupole form, forward and backward
+        // over 20 turns of the learnable FODO ring 8.26 -> 6.83 ms.
+        int64_t e = (int64_t)wl;
+        const uint64_t *rec = a.stream + a.elem_offset[e];
+        uint64_t hdr = rec[0], first = rec[1];
+        int64_t off = a.elem_offset[e > 0 ? e - 1 : 0];
+        int32_t j1 = a.pbeg ? a.pbeg[e + 1] : 0, j0 = a.pbeg ? a.pbeg[e] : 0;
+        for (; e >= 0; --e) {
+            const uint64_t *const next = a.stream + off;
+            uint64_t const next_hdr = next[0], next_first = next[1];
+            off = a.elem_offset[e > 1 ? e - 2 : 0];
+            int32_t const next_j0 = a.pbeg ? a.pbeg[e > 0 ? e - 1 : 0] : 0;
+            reverse_elem<BB6D>(s, l, rec, hdr, W(first), a, j0, j1, act && e <= mine);
+            rec = next;
+            hdr = next_hdr;
+            first = next_first;
+            j1 = j0;
+            j0 = next_j0;
+        }
     }
     if (part) {
         a.lam[0 * n + i] = l.x;
