@@ -10,6 +10,7 @@
 #include "lattice.h"
 
 #include "leadkick.cuh"
+#include "sckick.cuh"
 
 #include <algorithm>
 #include <array>
@@ -277,6 +278,14 @@ bool compile_lattice(const ImageView &img, uint64_t begin, uint64_t end,
                                             (1.0 / (2.0 * kPi * kEps0))
                                       : 0.0));
                 p.push_back(d2w(round ? 1.0 / sigma : 0.0));
+                if (abs_omq < 1e-6 && (round || ell) && p.size() == SC_PAIR_AT) {
+                    uint64_t blk[kScPairWords];
+                    double const line = w2d(w[4]) * w2d(w[0]) * (sqrt_beta / w2d(w[9]));
+                    if (sc_pair_block(line, sqrt_beta, round, sigma, sx, sy, blk)) {
+                        aux |= SC_PAIR;
+                        p.insert(p.end(), blk, blk + kScPairWords);
+                    }
+                }
             }
             break;
         case ST_OBJECT_TYPE_SC_INTERPOLATED_PROF: {

@@ -109,29 +109,38 @@ STG_HD FPair mul(FPair a, FPair b)
     return FPair{p, ffma(a.l, b.h, e)};
 }
 
+// A float as a double, 0 below the normal range.
+STG_HD double as_double(float v)
+{
+    uint32_t const w = w_of(v), a = w & 0x7FFFFFFFu;
+    return a < 0x00800000u ? 0.0 : from_words(((a >> 3) + 0x38000000u) | (w & 0x80000000u), w << 29);
+}
+
 // Doubles at or outside both ends of [h + l - d, h + l + d] (d with a slack
-// of a unit in their last place).  False where d is not small against h.
-STG_HD bool double_bounds(FPair v, float d, double *lo_v, double *hi_v)
+// of a unit in their last place).
+STG_HD void double_bounds(FPair v, float d, double *lo_v, double *hi_v)
 {
     float const h = fadd(v.h, v.l), l = fsub(v.l, fsub(h, v.h));
     uint32_t const w = w_of(h);
     uint32_t const sign = w & 0x80000000u, e = w & 0x7F800000u;
     // +-2^(52 - exponent): l in units of the last of 53 bits
     float const s = f_of((0x99000000u - e) | sign);
-    float const ds = fabs_(fmul(d, s));
-    int32_t const a = frint(fmul(fsub(l, d), s)), b = frint(fmul(fadd(l, d), s));
-    uint64_t const m = ((uint64_t)(((w & 0x7FFFFFFFu) >> 3) + 0x38000000u) << 32) | (w << 29);
-    uint64_t const sg = (uint64_t)sign << 32;
-    *lo_v = from_bits((m + (uint64_t)(int64_t)a) | sg);
-    *hi_v = from_bits((m + (uint64_t)(int64_t)b) | sg);
-    if (e < (52u << 23)) {  // below 2^-75, zeros included: within +-2^-74
-        bool const zero = (w << 1) == 0u && d == 0.0f;
-        *lo_v = zero ? 0.0 : -0x1p-74;
-        *hi_v = zero ? 0.0 : 0x1p-74;
-        return d < 0x1p-75f;
+    if (e >= (52u << 23) && fabs_(fmul(d, s)) < 0x1p29f && (w & 0x7FFFFFu) != 0u) {
+        int32_t const a = frint(fmul(fsub(l, d), s)), b = frint(fmul(fadd(l, d), s));
+        uint64_t const m =
+            ((uint64_t)(((w & 0x7FFFFFFFu) >> 3) + 0x38000000u) << 32) | (w << 29);
+        uint64_t const sg = (uint64_t)sign << 32;
+        *lo_v = from_bits((m + (uint64_t)(int64_t)a) | sg);
+        *hi_v = from_bits((m + (uint64_t)(int64_t)b) | sg);
+        return;
     }
-    // a power of two may have l of the other sign, in a binade of finer units
-    return ds < 0x1p29f && (w & 0x7FFFFFu) != 0u;
+    // a bound that is not small against h, a value below 2^-75, or a power of
+    // two (whose l may lie in a binade of finer units): to single precision
+    float const wide = (w << 1) == 0u && d == 0.0f
+                           ? 0.0f
+                           : fadd(fadd(fmul(d, 1.0078125f), fmul(fabs_(h), 0x1p-22f)), 0x1p-100f);
+    *lo_v = as_double(fsub(h, wide));
+    *hi_v = as_double(fadd(h, wide));
 }
 
 // Nearest integer of (h + l) with |h| < 2^42, and whether h + l stays more
@@ -230,9 +239,9 @@ STG_HD bool lead_exact(double x, double y, const uint64_t *bal, int order, doubl
     *u1 = from_bits(bal[2] + (uint64_t)i);
     FPair const ey = mul(v, t.y), ex = mul(v, t.x);
     float const d = fmul(fabs_(t.y.h), ffma(high_f(blk[2]), t.s.h, low_f(blk[2])));
-    bool const ok1 = double_bounds(ey, fmul(fabs_(t.y.h), d), &e1[0], &e1[1]);
-    bool const ok2 = double_bounds(ex, fmul(fabs_(t.x.h), d), &e2[0], &e2[1]);
-    return ok && ok1 && ok2;
+    double_bounds(ey, fmul(fabs_(t.y.h), d), &e1[0], &e1[1]);
+    double_bounds(ex, fmul(fabs_(t.x.h), d), &e2[0], &e2[1]);
+    return ok;
 }
 
 // c_1 = RN(RN(b_1 - s g_3) + 2x g_2) of the fast policy's Goertzel form, and
@@ -249,9 +258,9 @@ STG_HD bool lead_fast(double x, double y, const uint64_t *bal, int order, double
     bool const oka = nearest(FPair{fmul(a.h, scale2), fmul(a.l, scale2)}, d, &ia);
     bool const okb = nearest(FPair{fmul(b.h, scale), fmul(b.l, scale)}, d, &ib);
     *c1 = from_bits(bal[2] + (uint64_t)(ia - ib));
-    bool const okw = double_bounds(
-        mul(t.s, t.g2), fmul(t.s.h, ffma(high_f(blk[2]), t.s.h, low_f(blk[2]))), &w[0], &w[1]);
-    return oka && okb && okw;
+    double_bounds(mul(t.s, t.g2), fmul(t.s.h, ffma(high_f(blk[2]), t.s.h, low_f(blk[2]))), &w[0],
+                  &w[1]);
+    return oka && okb;
 }
 
 // ------------------------------------------------------------ host: the block

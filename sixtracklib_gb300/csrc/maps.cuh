@@ -17,6 +17,7 @@
 #include "exp_table.h"
 #include "intpath.cuh"
 #include "leadkick.cuh"
+#include "sckick.cuh"
 #include "stream.h"
 
 namespace stg {
@@ -1228,6 +1229,35 @@ static __device__ __noinline__ PState sc_qgauss(PState p, const uint64_t *rec, u
     p.px += fk * ex;
     p.py += fk * ey;
     return p;
+}
+
+// The momenta after a q-Gaussian kick evaluated in FP32 pairs (sckick.cuh);
+// not ok where its bound leaves a sum open.
+struct ScKick {
+    double px, py;
+    bool ok;
+};
+
+static __device__ __noinline__ ScKick sc_qgauss_pair(double x, double y, double px, double py,
+                                                     double zeta, double inv_rvv, double sc_k,
+                                                     const uint64_t *c, uint32_t aux)
+{
+    ScKick r{px, py, false};
+    const uint64_t *const blk = c + SC_PAIR_AT;
+    FPair const k = sc_factor(sc_k);
+    if (!__all_sync(__activemask(), sc_small(k, px, py, blk))) return r;
+    if ((c[5] | c[6]) << 1) {  // an offset beam
+        x = less(x, W(c[5]));
+        y = less(y, W(c[6]));
+    }
+    double kx[2], ky[2];
+    if (!sc_pair_kick(x, y, k, zeta, inv_rvv, blk, (aux & SC_ROUND) != 0u,
+                      (aux & SC_ELL_X) != 0u, kx, ky))
+        return r;
+    r.px = px + kx[0];
+    r.py = py + ky[0];
+    r.ok = same_bits(r.px, px + kx[1]) && same_bits(r.py, py + ky[1]);
+    return r;
 }
 
 // NS(LineDensityProfileData_interpolate_value), be_beamfields.h:3385-3408,

@@ -46,7 +46,9 @@ enum Op : uint32_t {
                             //  min_sigma_diff, sigma = (sigma_x + sigma_y) / 2;
                             // bit1 / bit2 (SC_ELL_X / SC_ELL_Y): elliptic with
                             //  sigma_x > sigma_y / sigma_x < sigma_y;
-                            // bit3 (SC_Q1): |1 - q| < 1e-6 (Gaussian profile)
+                            // bit3 (SC_Q1): |1 - q| < 1e-6 (Gaussian profile);
+                            // bit4 (SC_PAIR): followed by the 8 words of
+                            //  sckick.cuh
     OP_MONITOR = 17,        // [num_stores, start, skip, max_pid, min_pid, rolling,
                             //  turn_ordered, out_ptr, out_capacity]
     OP_NOP = 18,            // success, no effect (disabled beam-beam)
@@ -94,6 +96,8 @@ constexpr uint32_t SC_ROUND = 1u;
 constexpr uint32_t SC_ELL_X = 2u;
 constexpr uint32_t SC_ELL_Y = 4u;
 constexpr uint32_t SC_Q1 = 8u;
+constexpr uint32_t SC_PAIR = 16u;
+constexpr uint32_t SC_PAIR_AT = 25;  // parameter index of the sckick.cuh words
 
 // BB6D aux flag: the strong beam's Sigma matrix is round and uncoupled
 // (S11 = S33, S12 = S34, S22 = S44, S13 = S14 = S23 = S24 = 0) with

@@ -266,6 +266,15 @@ __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t
     case OP_SC_QGAUSS:
         if constexpr (KIND != KIND_FULL) break;
         else {
+            if (aux & SC_PAIR) {
+                ScKick const k = sc_qgauss_pair(p.x, p.y, p.px, p.py, p.zeta, p.inv_rvv, p.sc_k,
+                                                rec + 1, aux);
+                if (k.ok) {
+                    p.px = k.px;
+                    p.py = k.py;
+                    return PASSED;
+                }
+            }
             p = sc_qgauss<FAST>(p, rec, aux);
             return PASSED;
         }

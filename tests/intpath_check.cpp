@@ -1,5 +1,5 @@
-// Checks intpath.cuh and leadkick.cuh on the CPU: every value they decide has
-// the bits of the FP64 sequence it stands for.  argv: what, samples, seed.  Prints
+// Checks intpath.cuh, leadkick.cuh and sckick.cuh on the CPU: every value they
+// decide has the bits of the FP64 sequence it stands for.  argv: what, samples, seed.  Prints
 // "<samples> <undecided> <different>".
 #include <cmath>
 #include <cstdio>
@@ -7,7 +7,7 @@
 #include <cstring>
 #include <random>
 
-#include "leadkick.cuh"
+#include "sckick.cuh"
 
 using namespace stg;
 
@@ -101,6 +101,77 @@ static void lead(bool fast, double rms, double errors, long n, long *undecided, 
     }
 }
 
+// The Faddeeva function of the CERN algorithm in long double (x, y > 0).
+static void cerrf(double x, double y, long double *wr, long double *wi)
+{
+    bool const inner = x < 5.33 && y < 4.29;
+    double const q = inner ? (1.0 - y / 4.29) * std::sqrt(1.0 - (x / 5.33) * (x / 5.33)) : 0.0;
+    int const nc = inner ? 7 + (int)(23.0 * q) : 1, nu = inner ? 10 + (int)(21.0 * q) : 9;
+    long double const g = 1.6 * q, u = y + g, v = x;
+    long double q1r = 1, q1i = 0, q2r = 0, q2i = 0, ar = 0, ai = 0;
+    for (int n = nu; n > 0; --n) {
+        if (n <= nc) ar = ar * g + q1r, ai = ai * g + q1i;
+        long double const qr = u * q1r - v * q1i + 0.5L * n * q2r;
+        long double const qi = u * q1i + v * q1r + 0.5L * n * q2i;
+        q2r = q1r, q2i = q1i, q1r = qr, q1i = qi;
+    }
+    long double const c = 0.5L * 1.12837916709551L / (q1r * q1r + q1i * q1i);
+    *wr = (ar * q1r + ai * q1i) * c;
+    *wi = (ar * q1i - ai * q1r) * c;
+}
+
+// Space-charge kicks of a beam of sx by sy, particles of rms amp: whether
+// the bounds hold the kick, and the momenta it leads to.
+static void space_charge(double sx, double sy, double amp, long n, long *undecided,
+                         long *different)
+{
+    constexpr double pi = 3.14159265358979323846, eps0 = 8.854187817620e-12;
+    bool const round = sx == sy, wide_x = sx > sy;
+    double const sb = 1.0 / (std::sqrt(2.0) * 0.1), line = 0.1 * 1e11 * sb / std::sqrt(pi);
+    double const su = wide_x ? sx : sy, sv = wide_x ? sy : sx;
+    double const S = std::sqrt(2.0 * (su * su - sv * sv));
+    double const factor = line / (round ? 2.0 * pi * eps0 : 2.0 * eps0 * std::sqrt(pi) * S);
+    uint64_t blk[kScPairWords];
+    if (!sc_pair_block(line, sb, round, 0.5 * (sx + sy), sx, sy, blk)) {
+        *undecided = n;
+        return;
+    }
+    for (long i = 0; i < n; ++i) {
+        double const x = amp * normal(), y = amp * normal(), zeta = 0.05 * normal();
+        double const irv = 1.0 + 1e-6 * normal(), k0 = 3.9e-40 * (1.0 + 1e-3 * normal());
+        double const px = 1e-5 * normal(), py = 1e-5 * normal();
+        long double const z = (long double)zeta * irv;
+        long double const K = (long double)k0 * factor * expl(-(long double)sb * sb * z * z);
+        long double ex, ey;
+        if (round) {
+            long double const r2 = (long double)x * x + (long double)y * y;
+            long double const t = K * -expm1l(-0.5L * r2 / (sx * sx)) / r2;
+            ex = t * x, ey = t * y;
+        } else {
+            double const u = std::fabs(wide_x ? x : y), v = std::fabs(wide_x ? y : x);
+            long double a, b, c, d;
+            cerrf(u / S, v / S, &a, &b);
+            cerrf(sv / su * u / S, su / sv * v / S, &c, &d);
+            long double const e = expl(-0.5L * ((long double)u * u / (su * su) +
+                                                (long double)v * v / (sv * sv)));
+            long double const fu = K * (b - d * e), fv = K * (a - c * e);
+            ex = std::copysign((double)(wide_x ? fu : fv), x);
+            ey = std::copysign((double)(wide_x ? fv : fu), y);
+        }
+        FPair const k = sc_factor(k0);
+        double kx[2], ky[2];
+        if (!sc_small(k, px, py, blk) ||
+            !sc_pair_kick(x, y, k, zeta, irv, blk, round, wide_x, kx, ky) ||
+            px + kx[0] != px + kx[1] || py + ky[0] != py + ky[1]) {
+            ++*undecided;
+            continue;
+        }
+        bool const in = std::fmin(kx[0], kx[1]) <= ex && ex <= std::fmax(kx[0], kx[1]) &&
+                        std::fmin(ky[0], ky[1]) <= ey && ey <= std::fmax(ky[0], ky[1]);
+        if (!in || px + kx[0] != px + (double)ex || py + ky[0] != py + (double)ey) ++*different;
+    }
+}
+
 int main(int argc, char **argv)
 {
     if (argc < 4) return 2;
@@ -110,6 +181,13 @@ int main(int argc, char **argv)
     if (!strncmp(argv[1], "lead", 4)) {
         bool const fast = argv[1][5] == 'f', wide = strstr(argv[1], "wide") != nullptr;
         lead(fast, wide ? 5e-3 : 1e-3, wide ? 1e-2 : 1e-4, n, &undecided, &different);
+        printf("%ld %ld %ld\n", n, undecided, different);
+        return 0;
+    }
+    if (!strncmp(argv[1], "sc", 2)) {
+        double const amp = strstr(argv[1], "wide") ? 5e-3 : strstr(argv[1], "core") ? 2e-5 : 1e-3;
+        double const sy = strstr(argv[1], "round") ? 1e-3 : strstr(argv[1], "tall") ? 1.2e-3 : 0.3e-3;
+        space_charge(1e-3, sy, amp, n, &undecided, &different);
         printf("%ld %ld %ld\n", n, undecided, different);
         return 0;
     }

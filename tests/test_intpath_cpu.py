@@ -1,5 +1,5 @@
 """The integer- and FP32-pipe parts of the element maps (csrc/intpath.cuh,
-csrc/leadkick.cuh), on the CPU: every value they decide has the bits of the
+csrc/leadkick.cuh, csrc/sckick.cuh), on the CPU: every value they decide has the bits of the
 FP64 sequence they stand for."""
 
 import os
@@ -40,5 +40,16 @@ def test_lead_kick_has_the_fp64_bits(check, what):
     small errors and at 5 mm with errors 100 times larger."""
     n, undecided, different = check(what, 400_000, 11)
     print(f"{what}: {undecided} of {n} left to the FP64 sequence")
+    assert different == 0
+    assert undecided < n
+
+
+@pytest.mark.parametrize("beam", ["round", "tall", "flat"])
+@pytest.mark.parametrize("where", ["sigma", "wide", "core"])
+def test_space_charge_kick_within_its_bounds(check, beam, where):
+    """The pair evaluation's bounds hold the kick (the CERN algorithm's
+    Faddeeva function in long double), at 1, 5 and 0.02 sigma rms."""
+    n, undecided, different = check(f"sc {beam} {where}", 50_000, 5)
+    print(f"{beam} {where}: {undecided} of {n} left to the FP64 evaluation")
     assert different == 0
     assert undecided < n

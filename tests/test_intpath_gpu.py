@@ -1,5 +1,5 @@
 """The integer- and FP32-pipe parts of the element maps (csrc/intpath.cuh,
-csrc/leadkick.cuh) on the GPU,
+csrc/leadkick.cuh, csrc/sckick.cuh) on the GPU,
 bit for bit against the oracle (exact policy) and its restatement of the
 fast policy, at the edges of the ranges they decide."""
 
@@ -139,3 +139,51 @@ def test_lead_block_follows_the_parameters(oracles):
         cols = torch.from_numpy(p.block.copy().view(np.int64)).cuda()
         assert lat.tracker.track_until(cols, 1) == 0
         assert np.array_equal(cols.cpu().numpy().view(np.uint64), exp)
+
+
+@pytest.mark.parametrize("sigmas", [(1e-3, 1e-3), (1e-3, 1.2e-3), (1e-3, 0.3e-3)])
+@pytest.mark.parametrize("size", [2e-5, 1e-3, 6e-3])
+def test_space_charge_kick(oracles, sigmas, size):
+    """q-Gaussian kicks 1e-11 of the momenta (pairs) and of the momenta's size
+    (FP64), centred and offset: exact mode equal to the oracle, whose libm and
+    Faddeeva function differ by 1e-14 of a kick -- 1e-9 of the last bit of a
+    momentum where the pairs decide.  The last kick, of a beam 1e9 times as
+    intense, is held to 1e-12 of the largest."""
+    n = 1500
+    p = lattices.gaussian_particles(n, seed=8, sx=size, sy=size)
+    p.x[:20], p.y[20:40] = 0.0, 0.0
+    p.px[40:60], p.py[60:80] = 0.0, 1e-15
+    p.px[80:100] = 1e-18
+    e = Elements()
+    for k, (x_co, y_co) in enumerate([(0.0, 0.0), (1e-5, 0.0), (0.0, -2e-5), (0.0, 0.0)]):
+        e.SCQGaussProfile(number_of_particles=1e11 * (1 + k), bunchlength_rms=0.1,
+                          sigma_x=sigmas[0], sigma_y=sigmas[1], length=0.1, x_co=x_co, y_co=y_co,
+                          min_sigma_diff=1e-10, q_param=1.0, enabled=1)
+    small = p.block.copy().view(np.float64)
+    lost = slice(0, 100)  # momenta at or below the kick's size: no last bit to compare
+    import torch
+
+    from sixtracklib_gb300.device import DeviceTracker
+
+    exp = p.block.copy()
+    oracles["exact"].track_until(e.cbuffer.to_image(), exp, 1)
+    for mode in ("exact", "fast"):
+        cols = torch.from_numpy(p.block.copy().view(np.int64)).cuda()
+        assert DeviceTracker(e, f"mode={mode}").track_until(cols, 1) == 0
+        got = cols.cpu().numpy().view(np.uint64)
+        assert np.array_equal(got[:, 100:], exp[:, 100:])
+        kick = got[8:10, lost].view(np.float64) - small[8:10, lost]
+        ref = exp[8:10, lost].view(np.float64) - small[8:10, lost]
+        assert np.abs(kick - ref).max() <= 1e-12 * np.abs(ref).max()
+    strong = Elements()
+    strong.SCQGaussProfile(number_of_particles=1e20, bunchlength_rms=0.1, sigma_x=sigmas[0],
+                           sigma_y=sigmas[1], length=0.1, min_sigma_diff=1e-10, q_param=1.0,
+                           enabled=1)
+    exp = p.block.copy()
+    oracles["exact"].track_until(strong.cbuffer.to_image(), exp, 1)
+    cols = torch.from_numpy(p.block.copy().view(np.int64)).cuda()
+    assert DeviceTracker(strong, "mode=exact").track_until(cols, 1) == 0
+    got = cols.cpu().numpy().view(np.uint64)
+    ref = exp[8:10].view(np.float64) - small[8:10]
+    assert np.abs(got[8:10].view(np.float64) - exp[8:10].view(np.float64)).max() <= \
+        1e-12 * np.abs(ref).max()
