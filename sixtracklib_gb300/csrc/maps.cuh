@@ -104,6 +104,46 @@ __device__ __forceinline__ void refresh_kick_factors(PState &p)
     p.slip_lim = slip_limit(p.rvv);
 }
 
+// Comparisons on the integer pipe (an FP64 compare occupies the FP64 pipe
+// like an addition).  v < 0; v > 0; v == 0.
+__device__ __forceinline__ bool negative(double v)
+{
+    uint32_t const hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
+    return (int32_t)hi < 0 && ((hi << 1) | lo) != 0u &&
+           ((hi << 1) < 0xFFE00000u || ((hi << 1) == 0xFFE00000u && lo == 0u));
+}
+__device__ __forceinline__ bool positive(double v)
+{
+    uint32_t const hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
+    return (int32_t)hi >= 0 && (hi | lo) != 0u && (hi < 0x7FF00000u || (hi == 0x7FF00000u && lo == 0u));
+}
+__device__ __forceinline__ bool zero(double v)
+{
+    return (((uint32_t)__double2hiint(v) << 1) | (uint32_t)__double2loint(v)) == 0u;
+}
+// |v| < lim, as the floating-point comparison (false for a NaN)
+__device__ __forceinline__ bool abs_less(double v, double lim)
+{
+    uint64_t const a = (uint64_t)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+    uint64_t const l = (uint64_t)__double_as_longlong(lim);
+    return a < l && l <= 0x7FF0000000000000ull;
+}
+// (a >= 0) - (a < 0) as a double
+__device__ __forceinline__ double sgn(double a)
+{
+    uint32_t const hi = (uint32_t)__double2hiint(a), lo = (uint32_t)__double2loint(a);
+    bool const nan = (hi << 1) > 0xFFE00000u || ((hi << 1) == 0xFFE00000u && lo != 0u);
+    uint32_t const s = ((hi << 1) | lo) != 0u ? hi & 0x80000000u : 0u;
+    return __hiloint2double(nan ? 0 : (int)(s | 0x3FF00000u), 0);
+}
+// the integer part of 0 <= v < 32
+__device__ __forceinline__ int trunc_small(double v)
+{
+    uint32_t const hi = (uint32_t)__double2hiint(v);
+    int const e = (int)(hi >> 20) - 1023;
+    return e < 0 ? 0 : (int)(((hi & 0xFFFFFu) | 0x100000u) >> (20 - e));
+}
+
 // ------------------------------------------------------------------ energy
 // NS(Particles_add_to_energy_value): particles.h:5255-5297
 __device__ __forceinline__ void add_energy(PState &p, double de)
@@ -560,21 +600,53 @@ __constant__ double kHalfN[32] = {0.0,  0.5,  1.0,  1.5,  2.0,  2.5,  3.0,  3.5,
 // (within an ulp of the quotients; nc and nu can differ only where 23 q or
 // 21 q lies within an ulp of an integer), and the final complex division
 // takes rcp_fast.
-template <bool FAST = false>
-static __device__ __noinline__ void cerrf(double in_re, double in_im, double *w_re, double *w_im)
+// Comparisons, nc, nu and the outer region's scaling (powers of two) run on
+// the integer pipe, and that region's first step, from Q = 1 and 0, costs
+// nothing: 60 FP64 instructions instead of 100 there, the same bits.
+struct Cplx {
+    double re, im;
+};
+
+// The outer region for coordinates beyond 2^400 or not finite.
+static __device__ __noinline__ Cplx cerrf_far(double x, double y)
+{
+    double const a_const = 1.12837916709551;
+    double q1r = 1.0, q1i = 0.0, q2r = 0.0, q2i = 0.0;
+    int ex;
+    frexp(fmax(x, y), &ex);
+    double const is = ldexp(1.0, -ex);
+    double const is2 = is * is;
+    double const w0r = y * is, w0i = x * is;
+    for (int n = 9; n > 0; n--) {
+        double const hn = (0.5 * n) * is2;
+        double const qr = fma(w0r, q1r, fma(-w0i, q1i, hn * q2r));
+        double const qi = fma(w0r, q1i, fma(w0i, q1r, hn * q2i));
+        q2r = q1r;
+        q2i = q1i;
+        q1r = qr;
+        q1i = qi;
+    }
+    double const q1sq = fma(q1r, q1r, q1i * q1i);
+    double const inv = 0.5 * a_const * is / q1sq;
+    return Cplx{fma(q2r, q1r, q2i * q1i) * inv, fma(q2r, q1i, -q2i * q1r) * inv};
+}
+
+template <bool FAST>
+static __device__ __noinline__ Cplx cerrf_c(double in_re, double in_im)
 {
     double const a_const = 1.12837916709551;
     double const xlim = 5.33, ylim = 4.29;
     double const x = fabs(in_re), y = fabs(in_im);
     double wx, wy;
-    double q1r = 1.0, q1i = 0.0, q2r = 0.0, q2i = 0.0;  // Q(n+1), Q(n+2)
-    if (y < ylim && x < xlim) {
+    uint32_t const top = max((uint32_t)__double2hiint(x), (uint32_t)__double2hiint(y));
+    if (abs_less(y, ylim) && abs_less(x, xlim)) {
+        double q1r = 1.0, q1i = 0.0, q2r = 0.0, q2i = 0.0;  // Q(n+1), Q(n+2)
         double const xr = FAST ? x * (1.0 / xlim) : x / xlim;
         double const q = (1.0 - (FAST ? y * (1.0 / ylim) : y / ylim)) * sqrt(1.0 - xr * xr);
         double const q32 = 3.2 * q;
         double const inv_2h = 0.5 * q32;  // 0.5 / h
-        int const nc = 7 + (int)(23.0 * q);
-        int const nu = 10 + (int)(21.0 * q);
+        int const nc = 7 + trunc_small(23.0 * q);
+        int const nu = 10 + trunc_small(21.0 * q);
         double const w0r = y + inv_2h, w0i = x;
         double ar = 0.0, ai = 0.0;  // A(n)
         // nu <= 31: q <= 1 for y >= 0 and x >= 0 inside the region
@@ -599,18 +671,29 @@ static __device__ __noinline__ void cerrf(double in_re, double in_im, double *w_
         double const inv = FAST ? (0.5 * a_const) * rcp_fast(q1sq) : 0.5 * a_const / q1sq;
         wx = fma(ar, q1r, ai * q1i) * inv;
         wy = fma(ar, q1i, -ai * q1r) * inv;
+    } else if (top >= (1423u << 20)) {
+        Cplx const w = cerrf_far(x, y);
+        wx = w.re;
+        wy = w.im;
     } else {
-        // |w0| is unbounded here: Q(n) = s^(10-n) Q'(n) with s a power of two
-        // near |w0| (exact scaling), Q'(n) = (w0 / s) Q'(n+1) + (n / 2 s^2) Q'(n+2)
-        int ex;
-        frexp(fmax(x, y), &ex);
-        double const is = ldexp(1.0, -ex);
-        double const is2 = is * is;  // a power of two: every product below is exact
+        // |w0| is unbounded here: Q(n) = s^(10-n) Q'(n) with s = 2^ex the power
+        // of two above max(x, y) (exact scaling), Q'(n) = (w0 / s) Q'(n+1) +
+        // (n / 2 s^2) Q'(n+2)
+        int const ex = (int)(top >> 20) - 1022;
+        double const is = __hiloint2double((1023 - ex) << 20, 0);
+        auto hn = [&](double half_n) {
+            return __hiloint2double(__double2hiint(half_n) - ((2 * ex) << 20), 0);
+        };
         double const w0r = y * is, w0i = x * is;
-        for (int n = 9; n > 0; n--) {
-            double const hn = (0.5 * n) * is2;
-            double const qr = fma(w0r, q1r, fma(-w0i, q1i, hn * q2r));
-            double const qi = fma(w0r, q1i, fma(w0i, q1r, hn * q2i));
+        // Q'(9) = w0 / s, Q'(8)
+        double q2r = w0r, q2i = w0i;
+        double q1r = fma(w0r, w0r, fma(-w0i, w0i, hn(4.0)));
+        double q1i = fma(w0r, w0i, w0i * w0r);
+#pragma unroll
+        for (int n = 7; n > 0; n--) {
+            double const h = hn(0.5 * n);
+            double const qr = fma(w0r, q1r, fma(-w0i, q1i, h * q2r));
+            double const qi = fma(w0r, q1i, fma(w0i, q1r, h * q2i));
             q2r = q1r;
             q2i = q1i;
             q1r = qr;
@@ -622,30 +705,47 @@ static __device__ __noinline__ void cerrf(double in_re, double in_im, double *w_
         wx = fma(q2r, q1r, q2i * q1i) * inv;
         wy = fma(q2r, q1i, -q2i * q1r) * inv;
     }
-    if (y == 0.) wx = exp(-x * x);
-    if (in_im < 0.) {
+    if (zero(y)) wx = exp(-x * x);
+    if (negative(in_im)) {
         wx = 2.0 * exp(y * y - x * x) * cos(2.0 * x * y) - wx;
         wy = -2.0 * exp(y * y - x * x) * sin(2.0 * x * y) - wy;
-        if (in_re > 0.) wy = -wy;
-    } else if (in_re < 0.) {
+        if (positive(in_re)) wy = -wy;
+    } else if (negative(in_re)) {
         wy = -wy;
     }
-    *w_re = wx;
-    *w_im = wy;
+    return Cplx{wx, wy};
+}
+
+template <bool FAST = false>
+__device__ __forceinline__ void cerrf(double in_re, double in_im, double *w_re, double *w_im)
+{
+    Cplx const w = cerrf_c<FAST>(in_re, in_im);
+    *w_re = w.re;
+    *w_im = w.im;
 }
 
 // gauss_fields.h:56-208 (NS(get_Ex_Ey_Gx_Gy_gauss), centred: Delta = 0)
-static __device__ __noinline__ void fields_gauss(double x, double y, double sigma_x, double sigma_y,
-                                          double min_sigma_diff, int skip_gs, double *ex_p,
-                                          double *ey_p, double *gx_p, double *gy_p)
+struct Field {
+    double ex, ey, gx, gy;
+};
+
+// The round field's factor within 1e-10 m of the axis, out of line: selected
+// inline, its square root would be computed for every particle.
+static __device__ __noinline__ double near_axis(double r2, double k) { return k * sqrt(r2); }
+static __device__ __noinline__ double near_axis_over(double r2, double d) { return sqrt(r2) / d; }
+
+static __device__ __noinline__ Field fields_gauss_v(double x, double y, double sigma_x,
+                                                    double sigma_y, double min_sigma_diff,
+                                                    int skip_gs)
 {
     double ex, ey, gx = 0., gy = 0.;
-    if (fabs(sigma_x - sigma_y) < min_sigma_diff) {
+    double const ds = sigma_x - sigma_y;
+    if (abs_less(ds, min_sigma_diff)) {
         double const sigma = 0.5 * (sigma_x + sigma_y);
         double const r2 = x * x + y * y;
         double t;
-        if (r2 < 1e-20)
-            t = sqrt(r2) / (2. * kPiD * kEps0D * sigma);
+        if (abs_less(r2, 1e-20))
+            t = near_axis_over(r2, 2. * kPiD * kEps0D * sigma);
         else
             t = (1 - exp(-0.5 * r2 / (sigma * sigma))) / (2. * kPiD * kEps0D * r2);
         ex = t * x;
@@ -663,7 +763,7 @@ static __device__ __noinline__ void fields_gauss(double x, double y, double sigm
     } else {
         double const abx = fabs(x), aby = fabs(y);
         double S, fact, wz_re, wz_im, we_re, we_im, e;
-        if (sigma_x > sigma_y) {
+        if (positive(ds)) {
             S = sqrt(2. * (sigma_x * sigma_x - sigma_y * sigma_y));
             fact = 1. / (2. * kEps0D * kSqrtPiD * S);
             double const eta_re = sigma_y / sigma_x * abx;
@@ -673,7 +773,7 @@ static __device__ __noinline__ void fields_gauss(double x, double y, double sigm
             e = exp(-abx * abx / (2 * sigma_x * sigma_x) - aby * aby / (2 * sigma_y * sigma_y));
             ex = fact * (wz_im - we_im * e);
             ey = fact * (wz_re - we_re * e);
-        } else if (sigma_x < sigma_y) {
+        } else if (negative(ds)) {
             S = sqrt(2. * (sigma_y * sigma_y - sigma_x * sigma_x));
             fact = 1. / (2. * kEps0D * kSqrtPiD * S);
             double const eta_re = sigma_x / sigma_y * aby;
@@ -686,8 +786,8 @@ static __device__ __noinline__ void fields_gauss(double x, double y, double sigm
         } else {
             ex = ey = __longlong_as_double(0x7FF0000000000000ll);  // 1/0
         }
-        if (x < 0) ex = -ex;
-        if (y < 0) ey = -ey;
+        if (negative(x)) ex = -ex;
+        if (negative(y)) ey = -ey;
         if (!skip_gs) {
             double const s11 = sigma_x * sigma_x, s33 = sigma_y * sigma_y;
             gx = -1. / (2 * (s11 - s33)) *
@@ -700,12 +800,18 @@ static __device__ __noinline__ void fields_gauss(double x, double y, double sigm
                       (sigma_x / sigma_y * exp(-x * x / (2 * s11) - y * y / (2 * s33)) - 1.));
         }
     }
-    *ex_p = ex;
-    *ey_p = ey;
-    if (!skip_gs) {
-        *gx_p = gx;
-        *gy_p = gy;
-    }
+    return Field{ex, ey, gx, gy};
+}
+
+__device__ __forceinline__ void fields_gauss(double x, double y, double sigma_x, double sigma_y,
+                                             double min_sigma_diff, int skip_gs, double *ex_p,
+                                             double *ey_p, double *gx_p, double *gy_p)
+{
+    Field const f = fields_gauss_v(x, y, sigma_x, sigma_y, min_sigma_diff, skip_gs);
+    *ex_p = f.ex;
+    *ey_p = f.ey;
+    *gx_p = f.gx;
+    *gy_p = f.gy;
 }
 
 // be_beamfields/track.h:89-149
@@ -725,8 +831,6 @@ static __device__ __noinline__ PState beam_beam_4d(PState p, const uint64_t *rec
     p.py += (fk * ey - W(d[9]));
     return p;
 }
-
-__device__ __forceinline__ double sgn(double a) { return (double)((a >= 0) - (a < 0)); }
 
 // be_beamfields/be_beamfields.h:2232-2385 (NS(BeamBeam6D_propagate_Sigma_matrix))
 // FAST (the general branch): one reciprocal of sqrt(T) for the three
@@ -757,7 +861,7 @@ static __device__ __noinline__ void bb6d_sigma(const uint64_t *sg, double S, dou
     double const dS_T = 2 * R * dS_R + 8. * S13 * dS_S13;
     double s11h, s33h, ct, st, ds11h, ds33h, dct, dst, c2t, dc2t;
     double const signR = sgn(R);
-    if (T < thr) {
+    if (abs_less(T, thr)) {
         double const a = S12 - S34;
         double const b = S22 - S44;
         double const c = S14 + S23;
@@ -803,7 +907,7 @@ static __device__ __noinline__ void bb6d_sigma(const uint64_t *sg, double S, dou
         s33h = 0.5 * (Wv - signR * sqrtT);
         dc2t = signR * (dS_R * isT - R * (0.5 * isT * isT * isT) * dS_T);
         dct = 0.25 * rcp_fast(ct) * dc2t;
-        if (fabs(st) < thr)
+        if (abs_less(st, thr))
             dst = (S14 + S23) / R;
         else
             dst = -0.25 * rcp_fast(st) * dc2t;
@@ -818,7 +922,7 @@ static __device__ __noinline__ void bb6d_sigma(const uint64_t *sg, double S, dou
         s33h = 0.5 * (Wv - signR * sqrtT);
         dc2t = signR * (dS_R / sqrtT - R / (2 * sqrtT * sqrtT * sqrtT) * dS_T);
         dct = 1. / (4. * ct) * dc2t;
-        if (fabs(st) < thr)
+        if (abs_less(st, thr))
             dst = (S14 + S23) / R;
         else
             dst = -1. / (4. * st) * dc2t;
@@ -851,7 +955,7 @@ __device__ __forceinline__ void fields_round_g_fast(double x, double y, double s
     double const r2 = x * x + y * y;
     double const inv_r2 = rcp_fast(r2);
     double const e = exp_fast(-0.5 * r2 * inv_s2);
-    double const t = (r2 < 1e-20) ? k * sqrt(r2 * inv_s2) : (1 - e) * k * inv_r2;
+    double const t = abs_less(r2, 1e-20) ? near_axis(r2 * inv_s2, k) : (1 - e) * k * inv_r2;
     double const exv = t * x, eyv = t * y;
     double const c = k * inv_s2;
     double const h = 0.5 * inv_r2;
@@ -866,8 +970,11 @@ __device__ __forceinline__ void fields_round_g(double x, double y, double sigma,
 {
     double const r2 = x * x + y * y;
     double const e = exp(-0.5 * r2 / (sigma * sigma));
-    double const t = (r2 < 1e-20) ? sqrt(r2) / (2. * kPiD * kEps0D * sigma)
-                                  : (1 - e) / (2. * kPiD * kEps0D * r2);
+    double t;
+    if (abs_less(r2, 1e-20))
+        t = near_axis_over(r2, 2. * kPiD * kEps0D * sigma);
+    else
+        t = (1 - e) / (2. * kPiD * kEps0D * r2);
     double const exv = t * x, eyv = t * y;
     double const c = 1. / (2 * kPiD * kEps0D * sigma * sigma);
     double const h = 1 / (2. * r2);
@@ -884,16 +991,16 @@ __device__ __forceinline__ void fields_round_g(double x, double y, double sigma,
 // function's fast form, and one exponential for the field and the G terms
 // (the reference evaluates the same exponent twice).  Within a few ulp of
 // fields_gauss.
-static __device__ __noinline__ void fields_gauss_fast(double x, double y, double sxx, double syy,
-                                                      double min_sigma_diff, double *ex_p,
-                                                      double *ey_p, double *gx_p, double *gy_p)
+static __device__ __noinline__ Field fields_gauss_fast(double x, double y, double sxx, double syy,
+                                                       double min_sigma_diff)
 {
     double const isx = rsqrt(sxx), isy = rsqrt(syy);
     double const sx = sxx * isx, sy = syy * isy;
-    if (fabs(sx - sy) < min_sigma_diff) {
+    if (abs_less(sx - sy, min_sigma_diff)) {
         double const sigma = 0.5 * (sx + sy);
-        fields_round_g_fast(x, y, sigma * sigma, ex_p, ey_p, gx_p, gy_p);
-        return;
+        Field f;
+        fields_round_g_fast(x, y, sigma * sigma, &f.ex, &f.ey, &f.gx, &f.gy);
+        return f;
     }
     constexpr double kFact = 1. / (2. * kEps0D * kSqrtPiD);
     constexpr double kG = 1. / (2 * kPiD * kEps0D);
@@ -902,16 +1009,17 @@ static __device__ __noinline__ void fields_gauss_fast(double x, double y, double
     double const e = exp_fast(-0.5 * (rx * rx + ry * ry));
     double ex, ey, i2;
     double wz_re, wz_im, we_re, we_im;
-    if (sxx > syy) {  // the branches on the variances: 2 (sxx - syy) keeps its sign
-        double const iS = rsqrt(2. * (sxx - syy));  // 1 / S
+    double const dss = sxx - syy;  // the branches on the variances, by its sign
+    if (positive(dss)) {
+        double const iS = rsqrt(2. * dss);  // 1 / S
         double const fact = kFact * iS;
         cerrf<true>(abx * iS, aby * iS, &wz_re, &wz_im);
         cerrf<true>((sy * isx) * abx * iS, (sx * isy) * aby * iS, &we_re, &we_im);
         ex = fact * (wz_im - we_im * e);
         ey = fact * (wz_re - we_re * e);
         i2 = iS * iS;  // 1 / (2 (sxx - syy))
-    } else if (sxx < syy) {
-        double const iS = rsqrt(2. * (syy - sxx));
+    } else if (negative(dss)) {
+        double const iS = rsqrt(-2. * dss);
         double const fact = kFact * iS;
         cerrf<true>(aby * iS, abx * iS, &wz_re, &wz_im);
         cerrf<true>((sx * isy) * aby * iS, (sy * isx) * abx * iS, &we_re, &we_im);
@@ -922,13 +1030,11 @@ static __device__ __noinline__ void fields_gauss_fast(double x, double y, double
         ex = ey = __longlong_as_double(0x7FF0000000000000ll);  // 1/0
         i2 = ex;
     }
-    if (x < 0) ex = -ex;
-    if (y < 0) ey = -ey;
+    if (negative(x)) ex = -ex;
+    if (negative(y)) ey = -ey;
     double const xe = x * ex + y * ey;
-    *ex_p = ex;
-    *ey_p = ey;
-    *gx_p = -i2 * (xe + kG * ((sy * isx) * e - 1.));
-    *gy_p = i2 * (xe + kG * ((sx * isy) * e - 1.));
+    return Field{ex, ey, -i2 * (xe + kG * ((sy * isx) * e - 1.)),
+                 i2 * (xe + kG * ((sx * isy) * e - 1.))};
 }
 
 // be_beamfields/track.h:342-507 with NS(BeamBeam6D_boost / inv_boost)
@@ -1013,7 +1119,11 @@ static __device__ __noinline__ PState beam_beam_6d(PState p, const uint64_t *rec
             double const r2 = fma(xb, xb, yb * yb);
             double const inv_s2 = rcp_fast(s_hat);
             double const e = exp_fast(-0.5 * r2 * inv_s2);
-            double const t = (r2 < 1e-20) ? k * sqrt(r2 * inv_s2) : (1 - e) * k * rcp_fast(r2);
+            double t;
+            if (abs_less(r2, 1e-20))
+                t = near_axis(r2 * inv_s2, k);
+            else
+                t = (1 - e) * k * rcp_fast(r2);
             double const kt = Ksl * t;
             double const Fx = kt * xb, Fy = kt * yb;
             bool const on_axis = ((uint64_t)__double_as_longlong(r2) << 1) == 0u;
@@ -1054,12 +1164,11 @@ static __device__ __noinline__ PState beam_beam_6d(PState p, const uint64_t *rec
                 double const ybh = -xb * st + yb * ct;
                 double const dxbh = xb * sm[6] + yb * sm[7];
                 double const dybh = -xb * sm[7] + yb * sm[6];
-                double ex, ey, gx = 0.0, gy = 0.0;
-                if (FAST)
-                    fields_gauss_fast(xbh, ybh, sm[0], sm[1], msd, &ex, &ey, &gx, &gy);
-                else
-                    fields_gauss(xbh, ybh, sqrt(sm[0]), sqrt(sm[1]), msd, 0, &ex, &ey, &gx, &gy);
-                double const Fxh = Ksl * ex, Fyh = Ksl * ey, Gxh = Ksl * gx, Gyh = Ksl * gy;
+                Field const f =
+                    FAST ? fields_gauss_fast(xbh, ybh, sm[0], sm[1], msd)
+                         : fields_gauss_v(xbh, ybh, sqrt(sm[0]), sqrt(sm[1]), msd, 0);
+                double const Fxh = Ksl * f.ex, Fyh = Ksl * f.ey;
+                double const Gxh = Ksl * f.gx, Gyh = Ksl * f.gy;
                 Fx = Fxh * ct - Fyh * st;
                 Fy = Fxh * st + Fyh * ct;
                 Fz = 0.5 * (Fxh * dxbh + Fyh * dybh + Gxh * sm[4] + Gyh * sm[5]);
@@ -1152,8 +1261,11 @@ static __device__ __noinline__ PState sc_qgauss(PState p, const uint64_t *rec, u
         double const ez = exp_fast(-(W(c[12]) * z * z));
         double const x = p.x - W(c[5]), y = p.y - W(c[6]);
         double const r2 = fma(x, x, y * y);
-        double const fr = (r2 < 1e-20) ? sqrt(r2) * W(c[24])
-                                       : (1.0 - exp_fast(-r2 * W(c[15]))) * rcp_fast(r2);
+        double fr;
+        if (abs_less(r2, 1e-20))
+            fr = near_axis(r2, W(c[24]));
+        else
+            fr = (1.0 - exp_fast(-r2 * W(c[15]))) * rcp_fast(r2);
         double const g = (p.sc_k * W(c[23])) * (ez * fr);
         p.px = fma(g, x, p.px);
         p.py = fma(g, y, p.py);
@@ -1192,9 +1304,11 @@ static __device__ __noinline__ PState sc_qgauss(PState p, const uint64_t *rec, u
         if (aux & SC_ROUND) {
             double const x = p.x - W(c[5]), y = p.y - W(c[6]);
             double const r2 = x * x + y * y;
-            double const t = (r2 < 1e-20) ? sqrt(r2) * W(c[16])
-                                          : (1.0 - exp_fast(-r2 * W(c[15]))) *
-                                                (1.0 / (2. * kPiD * kEps0D)) * rcp_fast(r2);
+            double t;
+            if (abs_less(r2, 1e-20))
+                t = near_axis(r2, W(c[16]));
+            else
+                t = (1.0 - exp_fast(-r2 * W(c[15]))) * (1.0 / (2. * kPiD * kEps0D)) * rcp_fast(r2);
             ex = t * x;
             ey = t * y;
         } else if (aux & (SC_ELL_X | SC_ELL_Y)) {
@@ -1215,8 +1329,8 @@ static __device__ __noinline__ PState sc_qgauss(PState p, const uint64_t *rec, u
                 ey = fact * (wz_im - we_im * e);
                 ex = fact * (wz_re - we_re * e);
             }
-            if (x < 0) ex = -ex;
-            if (y < 0) ey = -ey;
+            if (negative(x)) ex = -ex;
+            if (negative(y)) ey = -ey;
         } else {
             fields_gauss(p.x - W(c[5]), p.y - W(c[6]), W(c[2]), W(c[3]), W(c[7]), 1, &ex, &ey,
                          &gx, &gy);

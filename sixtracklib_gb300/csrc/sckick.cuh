@@ -183,9 +183,10 @@ struct WPair {
 // call.
 STG_HD bool w_start(FPair x, FPair y, WPair *s)
 {
-    float const dx = fsub(x.h, 5.33f), dy = fsub(y.h, 4.29f);
+    float const dx = fadd(fsub(x.h, 0x1.551eb80000000p+2f), fsub(x.l, 0x1.47ae140000000p-24f));
+    float const dy = fadd(fsub(y.h, 0x1.128f5c0000000p+2f), fsub(y.l, 0x1.47ae140000000p-25f));
     bool const inner = dx < 0.0f && dy < 0.0f;
-    bool const edge = (fabs_(dx) < 1e-5f && dy < 1e-5f) || (fabs_(dy) < 1e-5f && dx < 1e-5f);
+    bool const edge = (fabs_(dx) < 1e-9f && dy < 1e-9f) || (fabs_(dy) < 1e-9f && dx < 1e-9f);
     s->x = x;
     s->q1r = FPair{1.0f, 0.0f};
     s->q1i = s->q2r = s->q2i = s->ar = s->ai = FPair{0.0f, 0.0f};
@@ -201,18 +202,22 @@ STG_HD bool w_start(FPair x, FPair y, WPair *s)
     float const r = fsqrt_(b.h);
     float const rl = fmul(fadd(ffma(-r, r, b.h), b.l), fmul(0.5f, frcp(r)));
     FPair const q = mul(add(one, neg(yr)), FPair{r, rl});
-    float const q23 = fmul(23.0f, q.h), q21 = fmul(21.0f, q.h);
-    int const ic = (int)q23, iu = (int)q21;
-    // distance of 23 q and 21 q from the integers at and above their floors
-    auto clear = [&](float k, int i) {
-        float const d = fadd(ffma(k, q.h, -(float)i), fmul(k, q.l));
-        return d > 0x1p-30f && d < 1.0f - 0x1p-24f;
+    // floors of 23 q and 21 q: a product rounded up to an integer (their
+    // last place is 2^-19) leaves a negative rest
+    auto floor_of = [&](float k, int *i) {
+        int const j = (int)fmul(k, q.h);
+        float const rest = fadd(ffma(k, q.h, -(float)j), fmul(k, q.l));
+        *i = rest < 0.0f ? j - 1 : j;
+        return fabs_(rest) > 0x1p-30f;
     };
+    int ic, iu;
+    bool const clear = floor_of(23.0f, &ic) && floor_of(21.0f, &iu);
+    if (!clear) return false;
     s->nc = 7 + ic;
     s->nu = 10 + iu;
     s->i2h = fmul(1.6f, q.h);
     s->w0r = add(y, FPair{s->i2h, 0.0f});
-    return !edge && clear(23.0f, ic) && clear(21.0f, iu);
+    return !edge;
 }
 
 // Step n in single floats (the low parts stay zero).
@@ -243,15 +248,38 @@ STG_HD void w_scale(WPair &s)
     s.ai.h = fmul(s.ai.h, down);
 }
 
-STG_HD void w_double(WPair &s, int n)
+// a b - c d + e f (f's low part zero) with one sum of the low parts: 30 operations.
+STG_HD FPair w_row(FPair a, FPair b, FPair c, FPair d, FPair e, float f)
 {
-    FPair const hn{fmul(0.5f, (float)n), 0.0f}, i2h{s.i2h, 0.0f};
-    if (n <= s.nc) {
-        s.ar = add(mul(s.ar, i2h), s.q1r);
-        s.ai = add(mul(s.ai, i2h), s.q1i);
+    float const p1 = fmul(a.h, b.h), p2 = fmul(c.h, d.h), p3 = fmul(e.h, f);
+    float const e1 = ffma(a.h, b.h, -p1), e2 = ffma(c.h, d.h, -p2), e3 = ffma(e.h, f, -p3);
+    FPair const s1 = two_sum(p1, -p2), s2 = two_sum(s1.h, p3);
+    float l = fadd(fadd(s1.l, s2.l), fadd(fsub(e1, e2), e3));
+    l = ffma(a.h, b.l, l);
+    l = ffma(a.l, b.h, l);
+    l = ffma(-c.h, d.l, l);
+    l = ffma(-c.l, d.h, l);
+    return renorm(s2.h, ffma(e.l, f, l));
+}
+
+// a g + q
+STG_HD FPair w_sum(FPair a, float g, FPair q)
+{
+    float const p = fmul(a.h, g), e = ffma(a.h, g, -p);
+    FPair const s = two_sum(p, q.h);
+    return FPair{s.h, fadd(fadd(s.l, e), ffma(a.l, g, q.l))};
+}
+
+// Step n in pairs.
+STG_HD void w_double(WPair &s, int n, bool series)
+{
+    float const hn = fmul(0.5f, (float)n);
+    if (series) {
+        s.ar = w_sum(s.ar, s.i2h, s.q1r);
+        s.ai = w_sum(s.ai, s.i2h, s.q1i);
     }
-    FPair const qr = add(mul_add_mul(s.w0r, s.q1r, neg(s.x), s.q1i), mul(s.q2r, hn));
-    FPair const qi = add(mul_add_mul(s.w0r, s.q1i, s.x, s.q1r), mul(s.q2i, hn));
+    FPair const qr = w_row(s.w0r, s.q1r, s.x, s.q1i, s.q2r, hn);
+    FPair const qi = w_row(s.w0r, s.q1i, neg(s.x), s.q1r, s.q2i, hn);
     s.q2r = s.q1r;
     s.q2i = s.q1i;
     s.q1r = qr;
@@ -282,9 +310,17 @@ STG_HD bool w_two(FPair x1, FPair y1, FPair x2, FPair y2, FPair *w1r, FPair *w1i
     }
     w_scale(a);
     w_scale(b);
+    // from m on both take every step: no branch between the four chains
+    int m = a.nc < b.nc ? a.nc : b.nc;
+    m = m < a.nu ? m : a.nu;
+    m = m < b.nu ? m : b.nu;
+    for (; n > m; --n) {
+        if (n <= a.nu) w_double(a, n, n <= a.nc);
+        if (n <= b.nu) w_double(b, n, n <= b.nc);
+    }
     for (; n > 0; --n) {
-        if (n <= a.nu) w_double(a, n);
-        if (n <= b.nu) w_double(b, n);
+        w_double(a, n, true);
+        w_double(b, n, true);
     }
     w_finish(a, w1r, w1i);
     w_finish(b, w2r, w2i);
@@ -319,14 +355,14 @@ STG_HD FPair sc_factor(double sc_k)
 }
 
 // Whether the kick is small enough for its bound to decide RN(p + k): the
-// largest field times the factors is below 2^-17 of both momenta.
+// largest field times the factors is below 2^-14 of both momenta.
 STG_HD bool sc_small(FPair k, double px, double py, const uint64_t *blk)
 {
     float const top = fmul(fmul(k.h, f_of((uint32_t)blk[0])), f_of((uint32_t)blk[1]));
     uint32_t const ax = (uint32_t)(bits_of(px) >> 32) & 0x7FFFFFFFu;
     uint32_t const ay = (uint32_t)(bits_of(py) >> 32) & 0x7FFFFFFFu;
     // top as the high word of a double, rounded up
-    uint32_t const t = (w_of(top) >> 3) + 0x38000001u + (17u << 20);
+    uint32_t const t = (w_of(top) >> 3) + 0x38000001u + (14u << 20);
     return top > 0x1p-110f && ax >= t && ay >= t && ax < 0x7FF00000u && ay < 0x7FF00000u;
 }
 
@@ -354,8 +390,8 @@ STG_HD bool sc_pair_kick(double x, double y, FPair k, double zeta, double inv_rv
         if (u.h < -80.0f) u = FPair{-80.0f, 0.0f};
         FPair const e = exp_pair(u), one = two_sum(1.0f, -e.h);
         FPair const g = mul(K, div(renorm(one.h, fsub(one.l, e.l)), r2));
-        // 1 - e to 2^-41 of 1, the rest to 2^-42 of itself
-        float const d = fmul(fmul(K.h, frcp(r2.h)), 0x1p-39f);
+        // e and the quotients to 2^-42 or better
+        float const d = fmul(fmul(K.h, frcp(r2.h)), 0x1p-41f);
         double_bounds(mul(X, g), fmul(fabs_(X.h), d), &kx[0], &kx[1]);
         double_bounds(mul(Y, g), fmul(fabs_(Y.h), d), &ky[0], &ky[1]);
         return true;
@@ -374,7 +410,7 @@ STG_HD bool sc_pair_kick(double x, double y, FPair k, double zeta, double inv_rv
     FPair const e = exp_pair(arg);
     FPair const fu = mul(K, add(w1i, neg(mul(w2i, e)))), fv = mul(K, add(w1r, neg(mul(w2r, e))));
     float const d = fmul(fmul(K.h, fadd(fadd(w1r.h, w1i.h), fmul(e.h, fadd(w2r.h, w2i.h)))),
-                         0x1p-40f);
+                         0x1p-41f);
     FPair fx = wide_x ? fu : fv, fy = wide_x ? fv : fu;
     if (X.h < 0.0f) fx = neg(fx);
     if (Y.h < 0.0f) fy = neg(fy);
@@ -395,9 +431,10 @@ inline bool sc_pair_block(double line, double sqrt_beta, bool round, double sigm
     double const S = std::sqrt(2.0 * (su * su - sv * sv));
     double const factor = std::ldexp(
         line * (round ? 1.0 / (2.0 * pi * eps0) : 1.0 / (2.0 * eps0 * sqrt_pi * S)), -90);
-    // the round field is at most 0.4513 / sigma, |w| at most 1
+    // the round field is at most 0.4513 / sigma; Re and Im of w, at most 1 and
+    // 0.61, bound the elliptic one
     double const words[kScPairWords] = {
-        factor, round ? 0.46 / sigma : 2.0, sqrt_beta * sqrt_beta,
+        factor, round ? 0.46 / sigma : 1.0, sqrt_beta * sqrt_beta,
         round ? 0.5 / (sigma * sigma) : 1.0 / S, round ? 0.0 : sv / su / S,
         round ? 0.0 : su / sv / S, round ? 0.0 : 0.5 / (su * su), round ? 0.0 : 0.5 / (sv * sv)};
     for (int k = 0; k < kScPairWords; ++k) {
