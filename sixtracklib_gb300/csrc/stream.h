@@ -31,7 +31,7 @@ enum Op : uint32_t {
     OP_RF_MULTIPOLE = 12,   // [voltage, frequency, lag, bal..., phase...] aux = order
     OP_BB4D = 13,           // [11 BB4D data words]
     OP_BB6D = 14,           // [34 head words, n_part[N], x[N], y[N], sigma[N]]
-                            // aux = N | BB6D_ROUND
+                            // aux = N | BB6D_ROUND | BB6D_UNCOUPLED
     OP_SC_COASTING = 15,    // [9 SCCoasting words]
     OP_SC_QGAUSS = 16,      // [11 SCQGaussProfile words, sqrt_beta = 1 / (sqrt(2)
                             //  bunchlength_rms), sqrt_beta^2, sqrt_beta / cq,
@@ -106,7 +106,12 @@ constexpr uint32_t SC_PAIR_AT = 25;  // parameter index of the sckick.cuh words
 // branch with cos theta = 1, sin theta = 0 and no theta derivative, and the
 // field is the round one: the map computes only what that branch needs.
 constexpr uint32_t BB6D_ROUND = 1u << 31;
-constexpr uint32_t BB6D_SLICES = BB6D_ROUND - 1u;
+// BB6D aux flag: uncoupled (S13 = S14 = S23 = S24 = 0) with threshold_singular
+// > 0.  Where R = S11 - S33 is not singular the propagation is S11(S) and
+// S33(S) themselves with cos theta = 1, sin theta = 0 and no theta derivative
+// (up to the rounding of the general formulas).
+constexpr uint32_t BB6D_UNCOUPLED = 1u << 30;
+constexpr uint32_t BB6D_SLICES = BB6D_UNCOUPLED - 1u;
 
 inline uint64_t make_header(uint32_t op, uint32_t nwords, uint32_t aux)
 {

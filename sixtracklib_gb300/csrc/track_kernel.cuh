@@ -252,9 +252,9 @@ __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t
         if constexpr (KIND != KIND_FULL) break;
         else {
             if (aux & BB6D_ROUND)
-                p = beam_beam_6d<true, FAST>(p, rec, (int)(aux & BB6D_SLICES));
+                p = beam_beam_6d<true, FAST>(p, rec, aux);
             else
-                p = beam_beam_6d<false, FAST>(p, rec, (int)aux);
+                p = beam_beam_6d<false, FAST>(p, rec, aux);
             return PASSED;
         }
     case OP_SC_COASTING:
