@@ -13,11 +13,12 @@
 // (computed per element by the lattice compiler, lead_block); where the
 // bound leaves a rounding open, the caller runs the FP64 sequence.
 //
-// FP64 instructions per kick of order n: fast 5 instead of 2n + 5, exact 8
-// instead of 7n - 3; about 130 FP32 and integer ones issue in their shadow.
+// FP64 instructions per kick of order n: fast 5 instead of 2n + 5, exact 4
+// instead of 7n - 3 (the corrections added on the significands of u_1 x and
+// u_1 y); about 130 FP32 and integer ones issue in their shadow.
 // Measured on the 20,000-element ring (orders 1 to 10): 1M polar-grid
 // protons, one turn, fast 222.9 -> 130.4 ms; 131,072 Gaussian ones, exact
-// 99.6 -> 41.7 ms.  For particles at 1 mm 0.02 % of the kicks are left to
+// 99.6 -> 34.5 ms.  For particles at 1 mm 0.02 % of the kicks are left to
 // the FP64 sequence.
 #pragma once
 
@@ -222,10 +223,11 @@ STG_HD float lead_error(const LeadTerms &t, uint64_t k)
     return fmul(fadd(fabs_(t.x.h), fabs_(t.y.h)), ffma(high_f(k), t.s.h, low_f(k)));
 }
 
-// u_1 = RN(b_1 + Re(z bracket)) of the exact policy, and bounds on
-// v_1 y and v_1 x, v_1 = Im(z bracket).  Returns whether u_1 is decided.
+// u_1 = RN(b_1 + Re(z bracket)) of the exact policy, the corrections v_1 y
+// and v_1 x, v_1 = Im(z bracket), and the bound on v_1 per coordinate.
+// Returns whether u_1 is decided.
 STG_HD bool lead_exact(double x, double y, const uint64_t *bal, int order, double *u1,
-                       double *e1, double *e2)
+                       FPair *e1, FPair *e2, float *bound)
 {
     const uint64_t *const blk = bal + 2 * order + 2;
     LeadTerms const t = lead_terms(x, y, blk, order);
@@ -237,11 +239,31 @@ STG_HD bool lead_exact(double x, double y, const uint64_t *bal, int order, doubl
     bool const ok =
         nearest(FPair{fmul(re.h, scale), fmul(re.l, scale)}, lead_error(t, blk[1]), &i);
     *u1 = from_bits(bal[2] + (uint64_t)i);
-    FPair const ey = mul(v, t.y), ex = mul(v, t.x);
+    *e1 = mul(v, t.y);
+    *e2 = mul(v, t.x);
     float const d = fmul(fabs_(t.y.h), ffma(high_f(blk[2]), t.s.h, low_f(blk[2])));
-    double_bounds(ey, fmul(fabs_(t.y.h), d), &e1[0], &e1[1]);
-    double_bounds(ex, fmul(fabs_(t.x.h), d), &e2[0], &e2[1]);
+    bound[0] = fmul(fabs_(t.y.h), d);
+    bound[1] = fmul(fabs_(t.x.h), d);
     return ok;
+}
+
+// RN(k + e), e known to +-d, formed on k's significand; false where the
+// rounding is open or the sum leaves k's binade.
+STG_HD bool nearest_sum(double k, FPair e, float d, double *sum)
+{
+    uint64_t const w = bits_of(k);
+    uint32_t const hi = (uint32_t)(w >> 32);
+    // e in units of k's last place, with k's sign: times +-2^(1075 - exponent)
+    uint32_t const ex = (hi >> 20) & 0x7FFu;
+    uint32_t const sb = ((1202u - ex) << 23) | (hi & 0x80000000u);
+    float const s = f_of(sb);
+    int64_t i;
+    // k between 2^-74 and 2^49, |e| below 2^41 of its last places
+    bool const fine = ex - 949u < 123u && fabs_(fmul(e.h, s)) < 0x1p41f;
+    bool const ok = nearest(FPair{fmul(e.h, s), fmul(e.l, s)}, fabs_(fmul(d, s)), &i);
+    uint64_t const r = w + (uint64_t)i;
+    *sum = from_bits(r);
+    return fine && ok && ((r ^ w) >> 52) == 0;
 }
 
 // c_1 = RN(RN(b_1 - s g_3) + 2x g_2) of the fast policy's Goertzel form, and

@@ -341,10 +341,27 @@ __device__ __forceinline__ bool same_bits(double a, double b)
     return __double2hiint(a) == __double2hiint(b) && __double2loint(a) == __double2loint(b);
 }
 
+// RN(v -+ RN(k + e)) with e known to +-d, from both ends of the bound; not ok
+// where these differ.
+struct Settled {
+    double v;
+    bool ok;
+};
+template <bool ADD>
+static __device__ __noinline__ Settled lead_settle(double v, double k, FPair e, float d)
+{
+    double b[2];
+    double_bounds(e, d, &b[0], &b[1]);
+    double const p = plus_zero(k + b[0]), q = plus_zero(k + b[1]);
+    double const r = ADD ? v + p : v - p;
+    return Settled{r, same_bits(r, ADD ? v + q : v - q)};
+}
+
 // The kick of a multipole with a lead block (leadkick.cuh); false where a
-// rounding is left open, with p unchanged.  u_1 x and u_1 y with the small
-// corrections are formed at both ends of their bounds; where these differ
-// the momenta still decide, being rounded more coarsely.  All lanes of the
+// rounding is left open, with p unchanged.  The small corrections to u_1 x
+// and u_1 y are added on their significands (exact) or at both ends of their
+// bounds (fast, and exact where the former leaves the rounding open); where
+// the ends differ the momenta still decide, being rounded more coarsely.  All lanes of the
 // warp in range or none (the others would run both sequences).
 template <bool FAST>
 __device__ __forceinline__ bool lead_kick(PState &p, const uint64_t *bal, int order)
@@ -363,14 +380,27 @@ __device__ __forceinline__ bool lead_kick(PState &p, const uint64_t *bal, int or
         p.px = px;
         p.py = fma(chi, dpy, p.py);
     } else {
-        double u1, e1[2], e2[2];
-        if (!lead_exact(x, y, bal, order, &u1, e1, e2)) return false;
+        double u1, sx, sy;
+        FPair e1, e2;
+        float d[2];
+        if (!lead_exact(x, y, bal, order, &u1, &e1, &e2, d)) return false;
         double const kx = u1 * x, ky = u1 * y;
-        double const a = plus_zero(kx - e1[0]), b = plus_zero(kx - e1[1]);
-        double const c = plus_zero(ky + e2[0]), d = plus_zero(ky + e2[1]);
-        double const px = p.px - a, py = p.py + c;
-        if (!same_bits(a, b) && !same_bits(px, less(p.px, b))) return false;
-        if (!same_bits(c, d) && !same_bits(py, less(p.py, -d))) return false;
+        FPair const m1{-e1.h, -e1.l};
+        double px, py;
+        if (nearest_sum(kx, m1, d[0], &sx)) {
+            px = p.px - sx;
+        } else {
+            Settled const r = lead_settle<false>(p.px, kx, m1, d[0]);
+            if (!r.ok) return false;
+            px = r.v;
+        }
+        if (nearest_sum(ky, e2, d[1], &sy)) {
+            py = p.py + sy;
+        } else {
+            Settled const r = lead_settle<true>(p.py, ky, e2, d[1]);
+            if (!r.ok) return false;
+            py = r.v;
+        }
         p.px = px;
         p.py = py;
     }

@@ -88,10 +88,19 @@ static void lead(bool fast, double rms, double errors, long n, long *undecided, 
                 }
                 rx = px - u;
                 ry = py + v;
-                double u1, e1[2], e2[2];
-                ok = ok && lead_exact(x, y, bal, order, &u1, e1, e2);
-                a = px - plus(u1 * x - e1[0]), b = px - plus(u1 * x - e1[1]);
-                c = py + plus(u1 * y + e2[0]), d = py + plus(u1 * y + e2[1]);
+                double u1, s1, s2, b1[2], b2[2];
+                FPair e1, e2;
+                float dd[2];
+                ok = ok && lead_exact(x, y, bal, order, &u1, &e1, &e2, dd);
+                double const kx = u1 * x, ky = u1 * y;
+                FPair const m1{-e1.h, -e1.l};
+                double_bounds(m1, dd[0], &b1[0], &b1[1]);
+                double_bounds(e2, dd[1], &b2[0], &b2[1]);
+                a = px - plus(kx + b1[0]), b = px - plus(kx + b1[1]);
+                c = py + plus(ky + b2[0]), d = py + plus(ky + b2[1]);
+                // formed on the significands: within the bounds
+                if (nearest_sum(kx, m1, dd[0], &s1)) a = b = px - s1;
+                if (nearest_sum(ky, e2, dd[1], &s2)) c = d = py + s2;
             }
             if (!ok || bits_of(a) != bits_of(b) || bits_of(c) != bits_of(d))
                 ++*undecided;
