@@ -206,6 +206,20 @@ static __device__ __noinline__ double drift_slip_fp64(double xp, double yp, doub
 
 static __device__ __noinline__ double drift_slip_large(int64_t v) { return scaled_53_large(v); }
 
+// a b: on the integer pipes (DENSE) or on the FP64 pipe.
+static __device__ __noinline__ double product(double a, double b) { return a * b; }
+template <bool DENSE>
+__device__ __forceinline__ double times(double a, double b)
+{
+    if constexpr (DENSE) {
+        double r;
+        if (!mul_rn(a, b, &r)) r = product(a, b);
+        return r;
+    } else {
+        return a * b;
+    }
+}
+
 // be_drift/track.h:45-67.  FAST keeps the reference's rounding of
 // 1 + (xp^2 + yp^2)/2 at the scale of 1.0: regrouping the zeta update as
 // L (rvv - 1) - (L/2)(xp^2 + yp^2) is more accurate but departs from the
@@ -214,11 +228,11 @@ static __device__ __noinline__ double drift_slip_large(int64_t v) { return scale
 // sequence's bits (drift_slip).
 // s is only accumulated when the turn did not start at s = +0 (otherwise it
 // comes from the lattice's s table).
-template <bool FAST, bool S_LIVE = true>
+template <bool FAST, bool S_LIVE, bool DENSE>
 __device__ __forceinline__ void drift(PState &p, double L)
 {
-    double const xp = p.px * p.rpp;
-    double const yp = p.py * p.rpp;
+    double const xp = times<DENSE>(p.px, p.rpp);
+    double const yp = times<DENSE>(p.py, p.rpp);
     if (FAST) {
         p.x = fma(xp, L, p.x);
         p.y = fma(yp, L, p.y);
@@ -363,7 +377,7 @@ static __device__ __noinline__ Settled lead_settle(double v, double k, FPair e, 
 // bounds (fast, and exact where the former leaves the rounding open); where
 // the ends differ the momenta still decide, being rounded more coarsely.  All lanes of the
 // warp in range or none (the others would run both sequences).
-template <bool FAST>
+template <bool FAST, bool DENSE>
 __device__ __forceinline__ bool lead_kick(PState &p, const uint64_t *bal, int order)
 {
     double const x = p.x, y = p.y, chi = p.chi;
@@ -374,7 +388,7 @@ __device__ __forceinline__ bool lead_kick(PState &p, const uint64_t *bal, int or
         double c1, w[2];
         if (!lead_fast(x, y, bal, order, &c1, w)) return false;
         double const a = fma(x, c1, -w[0]), b = fma(x, c1, -w[1]);
-        double const dpy = y * c1;
+        double const dpy = times<DENSE>(y, c1);
         double const px = fma(-chi, a, p.px);
         if (!same_bits(a, b) && !same_bits(px, less_product(p.px, chi, b))) return false;
         p.px = px;
@@ -384,7 +398,7 @@ __device__ __forceinline__ bool lead_kick(PState &p, const uint64_t *bal, int or
         FPair e1, e2;
         float d[2];
         if (!lead_exact(x, y, bal, order, &u1, &e1, &e2, d)) return false;
-        double const kx = u1 * x, ky = u1 * y;
+        double const kx = times<DENSE>(x, u1), ky = times<DENSE>(y, u1);
         FPair const m1{-e1.h, -e1.l};
         double px, py;
         if (nearest_sum(kx, m1, d[0], &sx)) {
@@ -407,13 +421,13 @@ __device__ __forceinline__ bool lead_kick(PState &p, const uint64_t *bal, int or
     return true;
 }
 
-template <bool FAST, bool CURV, bool LEAD>
+template <bool FAST, bool CURV, bool LEAD, bool DENSE>
 __device__ __forceinline__ void multipole(PState &p, const uint64_t *rec, uint32_t aux)
 {
     const uint64_t *bal = rec + 1;
     int const order = (int)(aux & MP_ORDER);
     if (LEAD && !CURV && (aux & MP_LEAD) && (!FAST || order >= 3))
-        if (lead_kick<FAST>(p, bal, order)) return;
+        if (lead_kick<FAST, DENSE>(p, bal, order)) return;
     double dpx = W(bal[2 * order]);
     double dpy = W(bal[2 * order + 1]);
     double const x = p.x, y = p.y, chi = p.chi;

@@ -192,7 +192,7 @@ enum Passed : int { PASSED = 0, LOST = 1, FAILED = -1 };
 // other opcode, so their fall-through (failure, particle lost, as for an
 // unknown type id) is never taken.  Maps that cannot lose a particle return a
 // constant, so the walk tests nothing after them.
-template <bool FAST, int KIND, bool S_LIVE>
+template <bool FAST, int KIND, bool S_LIVE, bool DENSE>
 __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t hdr,
                                         const TrackParams &prm, int64_t start_elem, int64_t ord)
 {
@@ -205,10 +205,10 @@ __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t
     };
     switch (op) {
     case OP_DRIFT:
-        drift<FAST, S_LIVE>(p, W(rec[1]));
+        drift<FAST, S_LIVE, DENSE>(p, W(rec[1]));
         return limit(!(aux & DRIFT_APERTURE) || inside_global(p, prm.xlim_bits, prm.ylim_bits));
     case OP_MULTIPOLE:
-        multipole<FAST, false, KIND != KIND_SIMPLE>(p, rec, aux);
+        multipole<FAST, false, KIND != KIND_SIMPLE, DENSE>(p, rec, aux);
         return PASSED;
     case OP_SROTATION:
         srotation<FAST>(p, rec);
@@ -223,7 +223,7 @@ __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t
         cavity(p, rec);
         return PASSED;
     case OP_MULTIPOLE_CURV:
-        multipole<FAST, true, false>(p, rec, aux);
+        multipole<FAST, true, false, false>(p, rec, aux);
         return PASSED;
     case OP_DRIFT_EXACT:
         drift_exact<S_LIVE>(p, W(rec[1]));
@@ -325,8 +325,9 @@ __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t
 // S_LIVE (block-uniform for the pass): some particle of the block
 // accumulates s, so drifts carry the s update.  EBE: element-by-element
 // output, whose particles may enter an element already lost (the reference
-// checks the state after the map).
-template <bool FAST, int KIND, bool S_LIVE, bool EBE>
+// checks the state after the map).  DENSE: some FP64 products on the integer
+// pipes (mul_rn).
+template <bool FAST, int KIND, bool S_LIVE, bool EBE, bool DENSE>
 __device__ __forceinline__ void walk_chunk(PState &p, const uint64_t *rec, const TrackParams &prm,
                                            bool &part, bool &active, int &status,
                                            int64_t &stop_elem, int64_t &ord, int64_t start_elem)
@@ -346,7 +347,7 @@ __device__ __forceinline__ void walk_chunk(PState &p, const uint64_t *rec, const
                 store_record(p, prm.ebe_out, prm.ebe_cap, j, ae, p.at_turn,
                              p.lazy_s ? prm.s_table[first + o] : p.s);
         }
-        Passed const rc = apply<FAST, KIND, S_LIVE>(p, rec, hdr, prm, start_elem, first + o);
+        Passed const rc = apply<FAST, KIND, S_LIVE, DENSE>(p, rec, hdr, prm, start_elem, first + o);
         if (rc != PASSED || (EBE && p.state != 1)) {
             if (rc == FAILED) status |= -1;
             part = false;
@@ -367,6 +368,15 @@ __device__ __forceinline__ void mbar_inval(uint64_t *bar)
     asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// Above two warps per scheduler (of 152 SMs) the FP64 pipe is the bound and
+// some of its multiplications run on the integer pipes beside it; below, a
+// warp's own chain of latencies is, and the FP64 instruction's 64 cycles are
+// the shorter way to a product.  Measured, integer against FP64 products: a
+// FODO ring, exact, 100,000 protons 2.00 against 2.72 ms, 60,000 1.22 / 1.41,
+// 32,000 0.75 / 0.77, 10,000 2.27 / 2.09 (more turns); a 2,000-element ring,
+// fast, 100,000 2.48 / 2.60, 32,000 1.16 / 1.15.
+constexpr int64_t kDenseParticles = 2 * 32 * 4 * 152;
+
 // One CTA's share of a tracking call: particle t of the launch (an index
 // into prm.idx, or prm.i0 + t).  Block-uniform control flow: every thread
 // walks every record of every chunk of every turn the block needs; lanes
@@ -375,8 +385,10 @@ __device__ __forceinline__ void mbar_inval(uint64_t *bar)
 // every copy it issued complete; the caller invalidates the barriers before
 // the shared memory is used again.
 template <bool FAST, int KIND>
-__device__ __forceinline__ void track_block(const TrackParams &prm, int64_t t, uint64_t *smem)
+__device__ __forceinline__ void track_block(const TrackParams &prm, int64_t t, uint64_t *smem,
+                                            int64_t together)
 {
+    bool const dense = together > kDenseParticles;
     int const stages = prm.stages;
     int const cw = prm.chunk_words;
     uint64_t *bars = smem;                 // `stages` mbarriers (8 B each, padded to 16 words)
@@ -469,14 +481,17 @@ __device__ __forceinline__ void track_block(const TrackParams &prm, int64_t t, u
             }
             const uint64_t *rec = bufs + (size_t)buf * cw;
             if (prm.mode == MODE_EBE)
-                walk_chunk<FAST, KIND, true, true>(p, rec, prm, part, active, status, stop_elem,
-                                                    ord, start_elem);
+                walk_chunk<FAST, KIND, true, true, false>(p, rec, prm, part, active, status,
+                                                          stop_elem, ord, start_elem);
             else if (s_live)
-                walk_chunk<FAST, KIND, true, false>(p, rec, prm, part, active, status, stop_elem,
-                                                     ord, start_elem);
+                walk_chunk<FAST, KIND, true, false, false>(p, rec, prm, part, active, status,
+                                                           stop_elem, ord, start_elem);
+            else if (dense)
+                walk_chunk<FAST, KIND, false, false, true>(p, rec, prm, part, active, status,
+                                                           stop_elem, ord, start_elem);
             else
-                walk_chunk<FAST, KIND, false, false>(p, rec, prm, part, active, status,
-                                                      stop_elem, ord, start_elem);
+                walk_chunk<FAST, KIND, false, false, false>(p, rec, prm, part, active, status,
+                                                            stop_elem, ord, start_elem);
             if (!resident) {
                 __syncthreads();  // every warp is done with this stage buffer
                 if (threadIdx.x == 0) {
@@ -569,7 +584,8 @@ template <bool FAST, int MIN_BLOCKS, int KIND>
 __global__ void __launch_bounds__(kMaxThreads, MIN_BLOCKS) track_kernel(TrackParams prm)
 {
     extern __shared__ __align__(128) uint64_t smem[];
-    track_block<FAST, KIND>(prm, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, smem);
+    track_block<FAST, KIND>(prm, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, smem,
+                            prm.idx ? *prm.count : prm.i1 - prm.i0);
 }
 
 // Persistent batched kernel: each CTA takes work items (a tile of
@@ -597,7 +613,7 @@ __global__ void __launch_bounds__(kMaxThreads, MIN_BLOCKS)
         prm.count = nullptr;
         prm.i0 = w.first;
         prm.i1 = (w.first + blockDim.x < prm.n) ? w.first + blockDim.x : prm.n;
-        track_block<FAST, KIND>(prm, threadIdx.x, smem);
+        track_block<FAST, KIND>(prm, threadIdx.x, smem, (int64_t)num_items * blockDim.x);
         __syncthreads();
         if (threadIdx.x == 0)
             for (int b = 0; b < prm.stages; ++b) mbar_inval(&smem[b]);

@@ -193,6 +193,28 @@ int main(int argc, char **argv)
         printf("%ld %ld %ld\n", n, undecided, different);
         return 0;
     }
+    if (!strncmp(argv[1], "product", 7)) {
+        for (long i = 0; i < n; ++i) {
+            double a, b;
+            if (strstr(argv[1], "bits")) {  // any bit pattern
+                a = from_bits(gen()), b = from_bits(gen());
+            } else if (strstr(argv[1], "short")) {  // exact and half-way products
+                a = std::ldexp((double)(int64_t)(gen() >> (10 + gen() % 50)), -40);
+                b = std::ldexp((double)(int64_t)(gen() >> (10 + gen() % 50)), -60);
+            } else if (strstr(argv[1], "special")) {
+                a = kSpecial[gen() % 13], b = kSpecial[gen() % 13];
+            } else {
+                a = real(-40, 2), b = 1.0 + real(-52, -2);
+            }
+            double r;
+            if (!mul_rn(a, b, &r))
+                ++undecided;
+            else if (bits_of(r) != bits_of(a * b))
+                ++different;
+        }
+        printf("%ld %ld %ld\n", n, undecided, different);
+        return 0;
+    }
     if (!strncmp(argv[1], "sc", 2)) {
         double const amp = strstr(argv[1], "wide") ? 5e-3 : strstr(argv[1], "core") ? 2e-5 : 1e-3;
         double const sy = strstr(argv[1], "round") ? 1e-3 : strstr(argv[1], "tall") ? 1.2e-3 : 0.3e-3;

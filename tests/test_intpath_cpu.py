@@ -53,3 +53,13 @@ def test_space_charge_kick_within_its_bounds(check, beam, where):
     print(f"{beam} {where}: {undecided} of {n} left to the FP64 evaluation")
     assert different == 0
     assert undecided < n
+
+
+@pytest.mark.parametrize("operands", ["ordinary", "bits", "short", "special"])
+def test_product_is_the_rounded_one(check, operands):
+    """mul_rn: significands of any length, halves, zeros of both signs,
+    subnormals, infinities and NaN (those it refuses)."""
+    n, undecided, different = check(f"product {operands}", 2_000_000, 3)
+    print(f"{operands}: {undecided} of {n} left to the FP64 product")
+    assert different == 0
+    assert undecided < n

@@ -187,3 +187,21 @@ def test_space_charge_kick(oracles, sigmas, size):
     ref = exp[8:10].view(np.float64) - small[8:10]
     assert np.abs(got[8:10].view(np.float64) - exp[8:10].view(np.float64)).max() <= \
         1e-12 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("mode", ["exact", "fast"])
+def test_products_on_the_integer_pipes(oracles, mode):
+    """More particles than two warps per scheduler (40,000): the products of
+    drifts and leading quadrupoles run on the integer pipes."""
+    px, py = _momenta()
+    n = 40_000
+    p = lattices.gaussian_particles(n, seed=6, sdelta=3e-3)
+    p.px[:] = np.resize(px, n)
+    p.py[:] = np.resize(py, n)
+    p.x[::7], p.y[::11] = 0.0, -0.0
+    e = Elements()
+    for k in range(6):
+        e.Drift(length=1.0 + k)
+        e.Multipole(knl=[0.0, 0.03 - 0.01 * k])
+        e.Multipole(knl=[0.0, 0.01 + 0.01 * k, 1e-6, 1e-7, -1e-8])
+    _same(e, p.block, oracles[mode], mode)
