@@ -39,6 +39,7 @@ namespace stg {
 struct Options {
     bool fast = false;
     int threads = 128;           // tracking kernel's block size (effective)
+    bool threads_given = false;  // set by the configuration: the launch does not choose
     int threads_general = 128;   // the reference's cuda.threads_per_block
     int track_threads_req = 0;   // cuda.track_threads_per_block as given (0: unset)
     int device = 0;
@@ -115,8 +116,10 @@ static bool parse_options(const char *cfg, Options *o, std::string *err)
                     else throw std::invalid_argument(v);
                 } else if (k == "threads_per_block" || k == "threads") {
                     o->threads_general = std::stoi(v);
+                    o->threads_given = true;
                 } else if (k == "track_threads_per_block") {
                     o->track_threads_req = std::stoi(v);
+                    o->threads_given = true;
                 } else if (k == "device" || k == "device_id") {
                     o->device = std::stoi(v);
                 } else if (k == "aperture") {
@@ -422,7 +425,8 @@ static int32_t run_track(Device *dev, const Options &opt, const DevStream &ds, u
     bool const segmented = wait && mode == MODE_UNTIL && i1 > i0 && seg < until_turn;
     while (i1 > i0) {
         prm.turn_cap = segmented ? (int32_t)std::min<int64_t>(seg, 2147483647) : 0;
-        int const rc = launch_track(prm, opt.fast, opt.threads, opt.blocks_per_sm, stream);
+        int const rc = launch_track(prm, opt.fast, opt.threads_given ? opt.threads : 0,
+                                    opt.blocks_per_sm, stream);
         if (rc != 0) {
             set_error(std::string("track kernel launch: ") + cudaGetErrorString((cudaError_t)rc));
             return -1;
@@ -450,6 +454,7 @@ static int32_t run_track(Device *dev, const Options &opt, const DevStream &ds, u
         if (*h_count == 0 || dev->h_flags[1] != 0) break;  // done, or a pipeline timeout
         prm.idx = idx;
         prm.count = count;
+        prm.live = *h_count;
         seg = segment_turns(*h_count, prm.num_elements);
     }
     if (!wait) return 0;
@@ -2223,7 +2228,7 @@ bool device_lattice_view(const st_DeviceLattice *L, LatticeLaunchView *v)
     v->n_chunks = L->full->cs.info.num_chunks;
     v->chunk_words = L->full->cs.info.chunk_words;
     v->stages = L->opt.stages;
-    v->threads = L->opt.threads;
+    v->threads = L->opt.threads_given ? L->opt.threads : 0;
     v->blocks_per_sm = L->opt.blocks_per_sm;
     v->num_elements = L->full->cs.info.num_elements;
     v->fast = L->opt.fast;

@@ -8,7 +8,7 @@
 namespace stg {
 
 constexpr int kMaxThreads = 256;  // largest block the kernels are built for
-constexpr int kDefaultStages = 4;
+constexpr int kDefaultStages = 3;
 
 enum TrackMode : int32_t { MODE_UNTIL = 0, MODE_LINE = 1, MODE_EBE = 2 };
 
@@ -67,12 +67,14 @@ struct TrackParams {
     EbeDevConfig ebe;
     const int64_t *idx;      // device: particle indices to track (null: i0..i1)
     const int64_t *count;    // device: number of entries of idx
+    int64_t live;            // host: that number where it is known (0: up to i1 - i0)
     const double *s_table;   // device: s before element k when a turn starts at s = 0
     uint32_t op_mask;        // opcodes present in the compiled range (stream.h)
 };
 
 // Launch one tracking kernel on `stream` (a cudaStream_t).  Returns the CUDA
 // error code of the launch (0 on success).
+// threads 0: chosen by the number of particles.
 // blocks_per_sm selects the register tier: 1 (up to 255 registers, no
 // spills) or 2 (at most 128 registers per thread, two CTAs per SM).
 // prm.op_mask selects the instantiation (lattice_kind).

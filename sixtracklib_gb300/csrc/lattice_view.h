@@ -12,7 +12,7 @@ struct LatticeLaunchView {
     const uint64_t *stream = nullptr;  // device: chunked element stream
     const double *s_table = nullptr;   // device: s table
     int32_t n_chunks = 0, chunk_words = 0, stages = 0;
-    int32_t threads = 0, blocks_per_sm = 1;
+    int32_t threads = 0, blocks_per_sm = 1;  // threads 0: the launch chooses
     int64_t num_elements = 0;
     bool fast = false;
     uint64_t xlim_bits = 0, ylim_bits = 0;
