@@ -26,6 +26,7 @@ HOST_SOURCES = ["buffer.cpp", "lattice.cpp", "output_buffer.cpp", "aliases.cpp"]
 CUDA_SOURCES = {
     "track_kernel.cu": ["-fmad=false"],
     "track_kernel_plain.cu": ["-fmad=false"],
+    "track_kernel_map.cu": ["-fmad=false"],
     "track_kernel_full.cu": ["-fmad=false"],
     "engine.cu": [],
     "probe.cu": [],

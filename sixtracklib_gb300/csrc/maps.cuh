@@ -145,14 +145,43 @@ __device__ __forceinline__ int trunc_small(double v)
 }
 
 // ------------------------------------------------------------------ energy
-// NS(Particles_add_to_energy_value): particles.h:5255-5297
-__device__ __forceinline__ void add_energy(PState &p, double de)
+// a / b from y = 1 / b correctly rounded: q = RN(a y), its remainder in one
+// fma, and q + remainder y rounds to the quotient (P. W. Markstein, IBM J.
+// Res. Dev. 34 (1990) 111; holds for every pair of 4- to 12-bit significands,
+// tried in full); three FP64 instructions where a division takes about nine.
+// Zeros and what is out of [2^-500, 2^500), where a product could leave the
+// normal range, take the division.
+static __device__ __noinline__ double quotient(double a, double b) { return a / b; }
+
+__device__ __forceinline__ bool mid_range(double v)
+{
+    uint32_t const e = ((uint32_t)__double2hiint(v) >> 20) & 0x7FFu;
+    return e - 523u < 1000u;
+}
+
+__device__ __forceinline__ double divide(double a, double b, double y)
+{
+    if (!(mid_range(a) && mid_range(y))) return quotient(a, b);
+    double const q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+
+// 1 / beta0 and 1 / energy0
+struct Recip {
+    double beta0, energy0;
+};
+
+// NS(Particles_add_to_energy_value): particles.h:5255-5297.  RECIP: the
+// divisions by beta0 and energy0 from their reciprocals.
+template <bool RECIP>
+__device__ __forceinline__ void add_energy(PState &p, double de, const Recip &inv)
 {
     double const beta0 = p.beta0;
     double const db0 = p.delta * beta0;
-    double const ptau_beta0 = de / p.energy0 + sqrt(db0 * db0 + 2.0 * db0 * beta0 + 1.0) - 1.0;
-    double const ptau = ptau_beta0 / beta0;
-    double const psigma = ptau / beta0;
+    double const den = RECIP ? divide(de, p.energy0, inv.energy0) : de / p.energy0;
+    double const ptau_beta0 = den + sqrt(db0 * db0 + 2.0 * db0 * beta0 + 1.0) - 1.0;
+    double const ptau = RECIP ? divide(ptau_beta0, beta0, inv.beta0) : ptau_beta0 / beta0;
+    double const psigma = RECIP ? divide(ptau, beta0, inv.beta0) : ptau / beta0;
     double const delta = sqrt(ptau * ptau + 2.0 * psigma + 1.0) - 1.0;
     double const opd = delta + 1.0;
     double const rvv = opd / (1.0 + ptau_beta0);
@@ -515,13 +544,14 @@ __device__ __forceinline__ void multipole(PState &p, const uint64_t *rec, uint32
 }
 
 // be_cavity/track.h:39-67 (rec: voltage, (2 pi / c) * frequency, deg2rad * lag)
-__device__ __forceinline__ void cavity(PState &p, const uint64_t *rec)
+template <bool RECIP>
+__device__ __forceinline__ void cavity(PState &p, const uint64_t *rec, const Recip &inv)
 {
     double const q = p.q0 * p.charge_ratio;
     double const tau = p.zeta / (p.beta0 * p.rvv);
     double const phase = W(rec[3]) - W(rec[2]) * tau;
     double const energy = q * W(rec[1]) * sin(phase);
-    add_energy(p, energy);
+    add_energy<RECIP>(p, energy, inv);
 }
 
 // be_srotation/track.h:38-69
@@ -610,7 +640,7 @@ static __device__ __noinline__ PState rf_multipole(PState p, const uint64_t *rec
     double const chi = p.chi;
     p.px += -chi * dpx;
     p.py += chi * dpy;
-    add_energy(p, cav_energy + rfm_energy);
+    add_energy<false>(p, cav_energy + rfm_energy, Recip{});
     return p;
 }
 
@@ -1525,27 +1555,74 @@ static __device__ __noinline__ PState sc_interpolated(PState p, const uint64_t *
 //          (i, then j, then k; each term ((c x^i) y^j) z^k times the power);
 //   fast:  the sums as nested Horner forms over z, y and x with FMAs, the
 //          derivative weights (2u, 3u^2) taken into the powers once.
+// The FP64 pipe bounds both.  The grid coordinates' signs, cells and fractions
+// are taken on the integer pipe (an FP64 floor, conversion or comparison
+// occupies the FP64 pipe): with the energy change from reciprocals, 65,536
+// protons x 2 turns of a ring with TriCubs, fast, 4.72 -> 3.76 ms.
+struct GridPoint {
+    int32_t i;
+    double frac;
+    bool inside;
+};
+
+// v = i + frac for 0 <= i <= top (top a count as a double, below 2^31)
+__device__ __forceinline__ GridPoint grid_point(double v, double top)
+{
+    uint32_t const hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
+    int const e = (int)((hi >> 20) & 0x7FFu) - 1023;
+    bool const none = ((hi << 1) | lo) == 0u;  // +-0
+    bool const sane = ((int32_t)hi >= 0 && e < 31) || none;  // not negative, NaN or huge
+    uint64_t const m = ((uint64_t)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
+    // bits below the point, left-aligned: below 1 the number itself
+    uint64_t const f = e < 0 ? 0ull : m << (12 + (e & 31));
+    int32_t const i = e < 0 ? 0 : (int32_t)(m >> (52 - (e & 31)));
+    uint32_t const fh = (uint32_t)(f >> 32), fl = (uint32_t)f;
+    int const z = fh ? __clz((int)fh) : 32 + __clz((int)fl);
+    uint64_t const n = f << (z & 63);  // leading bit at 63
+    uint32_t const nh = (uint32_t)(n >> 32);
+    double const frac =
+        f ? __hiloint2double((int)(((uint32_t)(1021 - z) << 20) + (nh >> 11)),
+                             (int)(((uint32_t)n >> 11) | (nh << 21)))
+          : 0.0;
+    uint32_t const th = (uint32_t)__double2hiint(top);
+    int const te = (int)((th >> 20) & 0x7FFu) - 1023;
+    // the integer top (0 <= top < 2^31, exact)
+    int64_t const tm = ((int64_t)((th & 0xFFFFFu) | 0x100000u) << 32) | (uint32_t)__double2loint(top);
+    int32_t const t = te < 0 ? ((th << 1) ? -1 : 0) : (int32_t)(tm >> (52 - (te & 31)));
+    return GridPoint{i, none ? 0.0 : (e < 0 ? v : frac), sane && (int32_t)th >= 0 && te < 31 && i <= t};
+}
+
+__device__ __forceinline__ double flip(double v, uint32_t sign)
+{
+    return __hiloint2double((int)((uint32_t)__double2hiint(v) ^ sign), __double2loint(v));
+}
+
+struct GridKick {
+    double px, py, energy;
+    bool inside;
+};
+
 template <bool FAST>
-static __device__ __noinline__ PState tricub(PState p, const uint64_t *rec, uint32_t aux)
+static __device__ __noinline__ GridKick tricub(double px, double py, double zeta, double beta0,
+                                               double rvv, double charge, double p0c, double x,
+                                               double y, const uint64_t *rec, uint32_t aux)
 {
     const uint64_t *c = rec + 1;
-    double const z = p.zeta / (p.beta0 * p.rvv);
-    double const fx = ((p.x - W(c[0])) - W(c[9])) * W(c[12]);
-    double const fy = ((p.y - W(c[1])) - W(c[10])) * W(c[13]);
+    double const z = zeta / (beta0 * rvv);
+    double const fx = ((x - W(c[0])) - W(c[9])) * W(c[12]);
+    double const fy = ((y - W(c[1])) - W(c[10])) * W(c[13]);
     double const fz = ((z - W(c[2])) - W(c[11])) * W(c[14]);
-    double const sign_x = ((aux & TRICUB_MIRROR_X) && fx < 0.0) ? -1. : 1.;
-    double const sign_y = ((aux & TRICUB_MIRROR_Y) && fy < 0.0) ? -1. : 1.;
-    double const sign_z = ((aux & TRICUB_MIRROR_Z) && fz < 0.0) ? -1. : 1.;
-    double const sfx = sign_x * fx, sfy = sign_y * fy, sfz = sign_z * fz;
-    double const ixf = floor(sfx), iyf = floor(sfy), izf = floor(sfz);
+    // the sign a mirrored axis takes out of its coordinate
+    uint32_t const sign_x = (aux & TRICUB_MIRROR_X) && negative(fx) ? 0x80000000u : 0u;
+    uint32_t const sign_y = (aux & TRICUB_MIRROR_Y) && negative(fy) ? 0x80000000u : 0u;
+    uint32_t const sign_z = (aux & TRICUB_MIRROR_Z) && negative(fz) ? 0x80000000u : 0u;
+    GridPoint const gx = grid_point(flip(fx, sign_x), W(c[15]));
+    GridPoint const gy = grid_point(flip(fy, sign_y), W(c[16]));
+    GridPoint const gz = grid_point(flip(fz, sign_z), W(c[17]));
     // inside the grid: 0 <= i <= n - 2 in every coordinate (NaN fails)
-    if (!(ixf >= 0.0 && ixf <= W(c[15]) && iyf >= 0.0 && iyf <= W(c[16]) && izf >= 0.0 &&
-          izf <= W(c[17]))) {
-        p.state = 0;
-        return p;
-    }
-    int64_t const ix = (int64_t)ixf, iy = (int64_t)iyf, iz = (int64_t)izf;
-    double const xn = sfx - ixf, yn = sfy - iyf, zn = sfz - izf;
+    if (!(gx.inside && gy.inside && gz.inside)) return GridKick{px, py, 0.0, false};
+    double const xn = gx.frac, yn = gy.frac, zn = gz.frac;
+    int64_t const ix = gx.i, iy = gy.i, iz = gz.i;
     const double *cf = reinterpret_cast<const double *>(c[20]) +
                        64 * (ix + (int64_t)c[18] * (iy + (int64_t)c[19] * iz));
     double kpx, kpy, kpt;
@@ -1610,19 +1687,30 @@ static __device__ __noinline__ PState tricub(PState p, const uint64_t *rec, uint
                     kpt += (double)k * (((__ldg(cf + k + 4 * j + 16 * i) * xp[i]) * yp[j]) * zp[k - 1]);
     }
     kpx *= W(c[6]);
-    kpx *= -sign_x;
+    kpx = flip(kpx, sign_x ^ 0x80000000u);
     kpx -= W(c[3]);
     kpy *= W(c[7]);
-    kpy *= -sign_y;
+    kpy = flip(kpy, sign_y ^ 0x80000000u);
     kpy -= W(c[4]);
     kpt *= W(c[8]);
-    kpt *= -sign_z;
+    kpt = flip(kpt, sign_z ^ 0x80000000u);
     kpt -= W(c[5]);
-    double const q = p.q0 * p.charge_ratio;
-    double const energy_kick = q * (p.p0c * kpt);
-    p.px += kpx;
-    p.py += kpy;
-    add_energy(p, energy_kick);
+    return GridKick{px + kpx, py + kpy, charge * (p0c * kpt), true};
+}
+
+// The whole element, for the kernel with every map.
+template <bool FAST>
+static __device__ __noinline__ PState tricub_element(PState p, const uint64_t *rec, uint32_t aux)
+{
+    GridKick const k = tricub<FAST>(p.px, p.py, p.zeta, p.beta0, p.rvv, p.q0 * p.charge_ratio,
+                                    p.p0c, p.x, p.y, rec, aux);
+    if (!k.inside) {
+        p.state = 0;
+        return p;
+    }
+    p.px = k.px;
+    p.py = k.py;
+    add_energy<false>(p, k.energy, Recip{});
     return p;
 }
 

@@ -8,6 +8,7 @@
 namespace stg {
 
 STG_KIND(extern, KIND_PLAIN)
+STG_KIND(extern, KIND_MAP)
 STG_KIND(extern, KIND_FULL)
 STG_KIND(, KIND_SIMPLE)
 
@@ -93,6 +94,8 @@ int launch_track(const TrackParams &params, bool fast, int threads, int blocks_p
         return launch_kind<KIND_SIMPLE>(prm, fast, two, blocks, threads, smem, s);
     case KIND_PLAIN:
         return launch_kind<KIND_PLAIN>(prm, fast, two, blocks, threads, smem, s);
+    case KIND_MAP:
+        return launch_kind<KIND_MAP>(prm, fast, two, blocks, threads, smem, s);
     default:
         return launch_kind<KIND_FULL>(prm, fast, two, blocks, threads, smem, s);
     }
@@ -107,6 +110,8 @@ int batch_ctas_per_sm(bool fast, LatticeKind kind, int threads, int blocks_per_s
         return (int)batch_occupancy_kind<KIND_SIMPLE>(fast, two, threads, smem, per_sm);
     case KIND_PLAIN:
         return (int)batch_occupancy_kind<KIND_PLAIN>(fast, two, threads, smem, per_sm);
+    case KIND_MAP:
+        return (int)batch_occupancy_kind<KIND_MAP>(fast, two, threads, smem, per_sm);
     default:
         return (int)batch_occupancy_kind<KIND_FULL>(fast, two, threads, smem, per_sm);
     }
@@ -120,6 +125,8 @@ int launch_batch(const BatchLaunch &b, void *stream)
         return launch_batch_kind<KIND_SIMPLE>(b, s);
     case KIND_PLAIN:
         return launch_batch_kind<KIND_PLAIN>(b, s);
+    case KIND_MAP:
+        return launch_batch_kind<KIND_MAP>(b, s);
     default:
         return launch_batch_kind<KIND_FULL>(b, s);
     }

@@ -1,5 +1,6 @@
 // track_kernel.cuh -- the tracking kernel (compiled by track_kernel.cu,
-// track_kernel_plain.cu and track_kernel_full.cu, one kind of lattice each).
+// track_kernel_plain.cu, track_kernel_map.cu and track_kernel_full.cu, one
+// kind of lattice each).
 //
 // One thread per particle; the particle's state lives in registers for the
 // whole call (all turns).  The compiled element stream is staged into shared
@@ -194,7 +195,8 @@ enum Passed : int { PASSED = 0, LOST = 1, FAILED = -1 };
 // constant, so the walk tests nothing after them.
 template <bool FAST, int KIND, bool S_LIVE, bool DENSE>
 __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t hdr,
-                                        const TrackParams &prm, int64_t start_elem, int64_t ord)
+                                        const TrackParams &prm, const Recip &inv, int64_t start_elem,
+                                        int64_t ord)
 {
     uint32_t const op = (uint32_t)(hdr & 0xFF);
     uint32_t const aux = (uint32_t)(hdr >> 32);
@@ -220,7 +222,7 @@ __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t
     case OP_LIMIT_ELLIPSE:
         return limit(inside_ellipse<FAST>(p, rec, aux));
     case OP_CAVITY:
-        cavity(p, rec);
+        cavity<KIND == KIND_MAP>(p, rec, inv);
         return PASSED;
     case OP_MULTIPOLE_CURV:
         multipole<FAST, true, false, false>(p, rec, aux);
@@ -285,10 +287,22 @@ __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t
             return PASSED;
         }
     case OP_TRICUB:
-        if constexpr (KIND != KIND_FULL) break;
-        else {
-            p = tricub<FAST>(p, rec, aux);
+        if constexpr (KIND == KIND_FULL) {
+            p = tricub_element<FAST>(p, rec, aux);
             return p.state == 1 ? PASSED : FAILED;  // outside the grid: lost, failure
+        } else if constexpr (KIND == KIND_MAP) {
+            GridKick const k = tricub<FAST>(p.px, p.py, p.zeta, p.beta0, p.rvv,
+                                            p.q0 * p.charge_ratio, p.p0c, p.x, p.y, rec, aux);
+            if (!k.inside) {
+                p.state = 0;
+                return FAILED;
+            }
+            p.px = k.px;
+            p.py = k.py;
+            add_energy<true>(p, k.energy, inv);
+            return PASSED;
+        } else {
+            break;
         }
     case OP_MONITOR: {
         uint64_t *out = reinterpret_cast<uint64_t *>(rec[8]);
@@ -329,7 +343,7 @@ __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t
 // pipes (mul_rn).
 template <bool FAST, int KIND, bool S_LIVE, bool EBE, bool DENSE>
 __device__ __forceinline__ void walk_chunk(PState &p, const uint64_t *rec, const TrackParams &prm,
-                                           bool &part, bool &active, int &status,
+                                           const Recip &inv, bool &part, bool &active, int &status,
                                            int64_t &stop_elem, int64_t &ord, int64_t start_elem)
 {
     if (!part) return;
@@ -347,7 +361,7 @@ __device__ __forceinline__ void walk_chunk(PState &p, const uint64_t *rec, const
                 store_record(p, prm.ebe_out, prm.ebe_cap, j, ae, p.at_turn,
                              p.lazy_s ? prm.s_table[first + o] : p.s);
         }
-        Passed const rc = apply<FAST, KIND, S_LIVE, DENSE>(p, rec, hdr, prm, start_elem, first + o);
+        Passed const rc = apply<FAST, KIND, S_LIVE, DENSE>(p, rec, hdr, prm, inv, start_elem, first + o);
         if (rc != PASSED || (EBE && p.state != 1)) {
             if (rc == FAILED) status |= -1;
             part = false;
@@ -405,8 +419,10 @@ __device__ __forceinline__ void track_block(const TrackParams &prm, int64_t t, u
         valid = i < prm.i1;
     }
     PState p;
+    Recip inv{};  // KIND_MAP
     if (valid) {
         load_particle(p, prm.cols, prm.n, i);
+        if constexpr (KIND == KIND_MAP) inv = Recip{1.0 / p.beta0, 1.0 / p.energy0};
         // s of a turn that starts at +0 comes from the lattice's s table
         p.lazy_s = (prm.mode != MODE_LINE) && (__double_as_longlong(p.s) == 0);
     }
@@ -481,16 +497,16 @@ __device__ __forceinline__ void track_block(const TrackParams &prm, int64_t t, u
             }
             const uint64_t *rec = bufs + (size_t)buf * cw;
             if (prm.mode == MODE_EBE)
-                walk_chunk<FAST, KIND, true, true, false>(p, rec, prm, part, active, status,
+                walk_chunk<FAST, KIND, true, true, false>(p, rec, prm, inv, part, active, status,
                                                           stop_elem, ord, start_elem);
             else if (s_live)
-                walk_chunk<FAST, KIND, true, false, false>(p, rec, prm, part, active, status,
+                walk_chunk<FAST, KIND, true, false, false>(p, rec, prm, inv, part, active, status,
                                                            stop_elem, ord, start_elem);
             else if (dense)
-                walk_chunk<FAST, KIND, false, false, true>(p, rec, prm, part, active, status,
+                walk_chunk<FAST, KIND, false, false, true>(p, rec, prm, inv, part, active, status,
                                                            stop_elem, ord, start_elem);
             else
-                walk_chunk<FAST, KIND, false, false, false>(p, rec, prm, part, active, status,
+                walk_chunk<FAST, KIND, false, false, false>(p, rec, prm, inv, part, active, status,
                                                             stop_elem, ord, start_elem);
             if (!resident) {
                 __syncthreads();  // every warp is done with this stage buffer

@@ -194,3 +194,49 @@ def test_adjoint_refuses_tricub(torch_cuda):
         else:
             with pytest.raises(RuntimeError, match="TriCub"):
                 lat.adjoint_turns(start, end, lam, 0, 2, grad)
+
+
+@pytest.mark.parametrize("voltages", [(0.0, 1e-290, 1e5), (1e308,), (np.inf,)])
+@pytest.mark.parametrize("mirror", [0, 1])
+@pytest.mark.parametrize("others", [False, True])
+def test_grid_edges_like_the_oracle(torch_cuda, oracle, others, mirror, voltages):
+    """Coordinates on the grid's nodes, one bit beside them, on both zeros,
+    past the last cell, huge and not finite, and cavities whose energy change
+    is zero, tiny, huge and infinite: exact mode bit-identical to the oracle, with
+    and without a beam-field element in the lattice (another kernel)."""
+    from sixtracklib_gb300.beam_elements import Elements
+    from sixtracklib_gb300.particles import Particles
+
+    rng = np.random.default_rng(7 + mirror)
+    step = 2.0**-9
+    e = Elements()
+    e.TriCub(data=1, length=0.5)
+    tc._grid(e, rng, 5, 6, 7, step, step, step, 0.0, 0.0, 0.0, mirror=(mirror,) * 3, scale=1e-7)
+    for u in voltages:
+        e.Cavity(voltage=u, frequency=4e8, lag=90.0)
+    if others:
+        e.SCCoasting(number_of_particles=0.0, circumference=1000.0, sigma_x=1e-3, sigma_y=1.5e-3)
+    img = e.cbuffer.to_image()
+    nodes = np.arange(-8, 9) * step
+    v = np.concatenate([nodes, np.nextafter(nodes, 1), np.nextafter(nodes, -1),
+                        rng.uniform(0, 4, 9) * step,
+                        [-0.0, 5e-324, -5e-324, 1e-300, 2.0**31 * step, 2.0**40, 1e300, -1e300,
+                         np.inf, -np.inf, np.nan]])
+    p = Particles.from_ref(num_particles=3 * len(v), p0c=450e9)
+    p.x[:], p.y[:], p.zeta[:] = 1.3 * step, 2.7 * step, 3.1 * step
+    p.particle_id[:] = np.arange(3 * len(v))
+    p.x[: len(v)] = v
+    p.y[len(v): 2 * len(v)] = v
+    p.zeta[2 * len(v):] = v * p.beta0[0]
+    exp = p.block.copy()
+    oracle.set_track_flags(2, 2, 2, 2)
+    try:
+        assert oracle.track_until(img, exp, 1) == -1
+    finally:
+        oracle.set_track_flags()
+    assert 20 < int((exp[20] == 1).sum()) < 3 * len(v) - 20
+    st, got = device(torch_cuda, img, p.block, f"mode=exact {ENABLED}", until=1)
+    assert st == -1
+    nan = np.isnan(exp[:17].view(np.float64)) & np.isnan(got[:17].view(np.float64))
+    np.testing.assert_array_equal(np.where(nan, 0, got[:17]), np.where(nan, 0, exp[:17]))
+    np.testing.assert_array_equal(got[17:], exp[17:])
