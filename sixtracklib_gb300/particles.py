@@ -92,20 +92,33 @@ class Particles:
         seg = self._words[off : off + self.num_particles]
         return seg.view(np.float64) if c < 17 else seg.view(np.int64)
 
+    def _view(self):
+        """The 21 x n column block in place, None when not contiguous."""
+        n = self.num_particles
+        offs = self._words[1 : 1 + NUM_COLUMNS].tolist()
+        if offs != [22 + c * n for c in range(NUM_COLUMNS)]:
+            return None
+        return self._words[22 : 22 + NUM_COLUMNS * n].reshape(NUM_COLUMNS, n)
+
     @property
     def block(self) -> np.ndarray:
         """The 21 x n column block as u64 words (a view when contiguous)."""
+        own = self._view()
+        if own is not None:
+            return own
         n = self.num_particles
-        offs = [int(self._words[1 + c]) for c in range(NUM_COLUMNS)]
-        if offs == [22 + c * n for c in range(NUM_COLUMNS)]:
-            return self._words[22 : 22 + NUM_COLUMNS * n].reshape(NUM_COLUMNS, n)
-        return np.stack([self._words[o : o + n] for o in offs])
+        return np.stack([self._words[o : o + n]
+                         for o in self._words[1 : 1 + NUM_COLUMNS].tolist()])
 
     def set_block(self, block: np.ndarray):
         block = np.asarray(block).reshape(NUM_COLUMNS, -1).view(np.uint64)
-        for c in range(NUM_COLUMNS):
-            off = int(self._words[1 + c])
-            self._words[off : off + self.num_particles] = block[c]
+        own = self._view()
+        if own is not None:
+            own[:] = block
+        else:
+            for c in range(NUM_COLUMNS):
+                off = int(self._words[1 + c])
+                self._words[off : off + self.num_particles] = block[c]
         if self._cbuffer is not None:
             self._cbuffer.touch()
 

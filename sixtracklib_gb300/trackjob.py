@@ -382,7 +382,7 @@ class TrackJob:
     def collect_particles(self):
         self._lib.st_TrackJob_collect_particles(self.ptr_st_track_job)
         for i in self._pset_indices:
-            cols = _c_columns(self._lib, self._c_particles.ptr, i)
+            cols = _c_view(self._lib, self._c_particles.ptr, i)
             self._particles_buffer.get_object(i).set_block(cols)
         self._particles_buffer.touch()
         return self
@@ -674,8 +674,8 @@ class TrackJob:
         ptr = self._lib.st_TrackJob_get_output_buffer(self.ptr_st_track_job)
         n = self._lib.st_Buffer_get_size(ptr)
         data = self._lib.st_Buffer_get_const_data_begin(ptr)
-        img = np.ctypeslib.as_array(C.cast(data, C.POINTER(C.c_uint64)), shape=(n // 8,)).copy()
-        self._output_buffer = CBuffer.from_image(img)
+        img = np.ctypeslib.as_array(C.cast(data, C.POINTER(C.c_uint64)), shape=(n // 8,))
+        self._output_buffer = CBuffer.from_image(img)  # copies every object
         self._output_buffer.typeids[TYPE_PARTICLE] = Particles
 
     def output_particles(self, index) -> Particles:
@@ -695,26 +695,28 @@ class st_ParticlesAddr(C.Structure):
             "at_element", "at_turn", "state")]
 
 
-class _StParticles(C.Structure):
-    _fields_ = [("num_particles", C.c_int64)] + [(f"c{i}", C.c_void_p) for i in range(21)]
+def _c_view(lib, c_buffer, index):
+    """The 21 columns of Particles object `index` of a C-side st_Buffer, in
+    place: one 21 x n array where they follow one another (the buffers lay
+    them out so), else a list of arrays."""
+    ptr = lib.st_Particles_buffer_get_particles(c_buffer, int(index))
+    if not ptr:
+        raise RuntimeError(f"object {index} is not a Particles object")
+    n, *addr = (C.c_uint64 * 22).from_address(ptr)
+    words = C.POINTER(C.c_uint64)
+    if n > 0 and addr == list(range(addr[0], addr[0] + 21 * 8 * n, 8 * n)):
+        return np.ctypeslib.as_array(C.cast(addr[0], words), shape=(21, n))
+    return [np.ctypeslib.as_array(C.cast(a, words), shape=(n,)) for a in addr]
 
 
 def _c_columns(lib, c_buffer, index, write=None):
     """Read (or overwrite) the 21 x n columns of Particles object `index` of a
     C-side st_Buffer."""
-    ptr = lib.st_Particles_buffer_get_particles(c_buffer, int(index))
-    if not ptr:
-        raise RuntimeError(f"object {index} is not a Particles object")
-    sp = _StParticles.from_address(ptr)
-    n = int(sp.num_particles)
-    out = np.empty((21, n), dtype=np.uint64)
-    for c in range(21):
-        col = np.ctypeslib.as_array(C.cast(getattr(sp, f"c{c}"), C.POINTER(C.c_uint64)), shape=(n,))
-        if write is not None:
-            col[:] = np.asarray(write[c]).view(np.uint64)
-        else:
-            out[c] = col
-    return out
+    cols = _c_view(lib, c_buffer, index)
+    if write is None:
+        return np.array(cols, dtype=np.uint64)
+    for col, new in zip([cols], [write]) if isinstance(cols, np.ndarray) else zip(cols, write):
+        col[:] = np.asarray(new).view(np.uint64)
 
 
 class CudaTrackJob(TrackJob):
