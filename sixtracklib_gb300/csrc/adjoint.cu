@@ -713,40 +713,45 @@ __device__ __forceinline__ void reverse_multipole(RState &s, Lam &l, const uint6
         multipole_grad<CURV>(x, y, chi * lpx, chi * lpy, hxl_l, hyl_l, a, j0, j1, on);
 }
 
-// Restore the input of one element from its output (state s) and apply
+// Drift (be_drift/track.h:45-67), 15 FP64 instructions.
+__device__ __forceinline__ void reverse_drift(RState &s, Lam &l, double L)
+{
+    // input from output: x -= L rpp px, zeta -= L (rvv - 1 - rpp^2 (px^2 + py^2) / 2)
+    double const px = s.px, py = s.py;
+    double const a_ = L * s.rpp;
+    s.x = fma(-a_, px, s.x);
+    s.y = fma(-a_, py, s.y);
+    s.zeta = fma(L, fma(s.hr2, fma(py, py, px * px), -s.rvvm1), s.zeta);
+    // lambda: d(out)/d(px, py, delta) with rpp(delta), rvv(delta) and
+    // q = l_xy - lz rpp p_xy:
+    //   l.px += L rpp qx, l.py likewise, l.d += L (drpp (px qx + py qy) + lz drvv)
+    double const qx = fma(-s.lzr, px, l.x), qy = fma(-s.lzr, py, l.y);
+    l.px = fma(a_, qx, l.px);
+    l.py = fma(a_, qy, l.py);
+    l.d = fma(L, fma(s.drpp, fma(py, qy, px * qx), s.lzdrvv), l.d);
+}
+
+__device__ __forceinline__ bool is_quadrupole(uint64_t hdr)
+{
+    constexpr uint32_t kMask = MP_ORDER | MP_SKEW0 | MP_DIPOLE0;
+    return (uint32_t)(hdr & 0xFF) == OP_MULTIPOLE &&
+           ((uint32_t)(hdr >> 32) & kMask) == (1u | MP_SKEW0 | MP_DIPOLE0);
+}
+
+// Restore the input of one element (not a drift or a quadrupole, which the
+// walk does itself) from its output (state s) and apply
 // lambda <- J^T lambda at that input.  `on` is false for lanes that do not
-// take part (they still join the warp reductions); `first` is the record's
-// first parameter, [j0, j1) its entries of the parameter list.  The 6D beam-beam
+// take part (they still join the warp reductions); [j0, j1) are its entries of
+// the parameter list.  The 6D beam-beam
 // reverse is compiled in only where BB6D is set: its call site alone costs
 // lattices without the element a few percent (registers saved around it).
 template <bool BB6D>
 __device__ __forceinline__ void reverse_elem(RState &s, Lam &l, const uint64_t *rec, uint64_t hdr,
-                                             double first, const AdjParams &a, int32_t j0,
-                                             int32_t j1, bool on)
+                                             const AdjParams &a, int32_t j0, int32_t j1, bool on)
 {
     uint32_t const op = (uint32_t)(hdr & 0xFF);
     uint32_t const aux = (uint32_t)(hdr >> 32);
     switch (op) {
-    case OP_DRIFT: {  // be_drift/track.h:45-67
-        if (!on) break;
-        // input from output: x -= L rpp px, zeta -= L (rvv - 1 - rpp^2 (px^2 + py^2) / 2)
-        double const L = first;
-        double const px = s.px, py = s.py;
-        double const a_ = L * s.rpp;
-        s.x = fma(-a_, px, s.x);
-        s.y = fma(-a_, py, s.y);
-        double const p2 = fma(py, py, px * px);
-        s.zeta = fma(L, fma(s.hr2, p2, -s.rvvm1), s.zeta);
-        // lambda: d(out)/d(px, py, delta) with rpp(delta), rvv(delta):
-        //   l.px += L rpp (lx - lz rpp px), l.py likewise,
-        //   l.d += L (drpp (lx px + ly py - lz rpp (px^2 + py^2)) + lz drvv)
-        double const lx = l.x, ly = l.y;
-        l.px = fma(a_, fma(-s.lzr, px, lx), l.px);
-        l.py = fma(a_, fma(-s.lzr, py, ly), l.py);
-        double const s1 = fma(ly, py, lx * px);
-        l.d = fma(L, fma(s.drpp, fma(-s.lzr, p2, s1), s.lzdrvv), l.d);
-        break;
-    }
     case OP_DRIFT_EXACT: {  // be_drift/track.h:71-97
         if (!on) break;
         double const L = W(rec[1]);
@@ -768,10 +773,7 @@ __device__ __forceinline__ void reverse_elem(RState &s, Lam &l, const uint64_t *
         break;
     }
     case OP_MULTIPOLE:  // be_multipole/track.h:38-112
-        if ((aux & (MP_ORDER | MP_SKEW0 | MP_DIPOLE0)) == (1u | MP_SKEW0 | MP_DIPOLE0))
-            reverse_quadrupole(s, l, W(rec[3]), a, j0, j1, on);
-        else
-            reverse_multipole<false>(s, l, rec + 1, (int)(aux & MP_ORDER), a, j0, j1, on);
+        reverse_multipole<false>(s, l, rec + 1, (int)(aux & MP_ORDER), a, j0, j1, on);
         break;
     case OP_MULTIPOLE_CURV:
         reverse_multipole<true>(s, l, rec + 1, (int)(aux & MP_ORDER), a, j0, j1, on);
@@ -912,28 +914,62 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm) adjoint_kernel(A
             long long const v = __shfl_xor_sync(0xFFFFFFFFu, wl, o);
             wl = v > wl ? v : wl;
         }
-        // The walk reads ahead: the offset of the record two elements on,
-        // the header, first parameter and parameter-list entry of the next.
-        // With one warp per scheduler (16,384 particles) an element's time
-        // was its chain of three dependent global reads plus its FP64
-        // instructions; with the short quadrupole form, forward and backward
-        // over 20 turns of the learnable FODO ring 8.26 -> 6.83 ms.
-        int64_t e = (int64_t)wl;
-        const uint64_t *rec = a.stream + a.elem_offset[e];
-        uint64_t hdr = rec[0], first = rec[1];
-        int64_t off = a.elem_offset[e > 0 ? e - 1 : 0];
-        int32_t j1 = a.pbeg ? a.pbeg[e + 1] : 0, j0 = a.pbeg ? a.pbeg[e] : 0;
-        for (; e >= 0; --e) {
-            const uint64_t *const next = a.stream + off;
-            uint64_t const next_hdr = next[0], next_first = next[1];
-            off = a.elem_offset[e > 1 ? e - 2 : 0];
-            int32_t const next_j0 = a.pbeg ? a.pbeg[e > 0 ? e - 1 : 0] : 0;
-            reverse_elem<BB6D>(s, l, rec, hdr, W(first), a, j0, j1, act && e <= mine);
-            rec = next;
-            hdr = next_hdr;
-            first = next_first;
-            j1 = j0;
-            j0 = next_j0;
+        // 32-bit element numbers below the multiple `lo` of 2^30
+        for (int64_t hi = (int64_t)wl, lo; hi >= 0; hi = lo - 1) {
+            lo = hi & ~(int64_t)0x3fffffff;
+            int32_t const last = mine < lo ? -1 : (int32_t)(mine < hi ? mine - lo : hi - lo);
+            const int64_t *const offsets = a.elem_offset + lo;
+            const int32_t *const pbeg = a.pbeg ? a.pbeg + lo : nullptr;
+            // The walk reads ahead: the offset of the record two elements on,
+            // the header, first parameter and parameter-list entry of the next.
+            // With one warp per scheduler (16,384 particles) an element's time
+            // was its chain of three dependent global reads plus its FP64
+            // instructions; with the short quadrupole form, forward and backward
+            // over 20 turns of the learnable FODO ring 8.26 -> 6.83 ms.
+            int32_t e = (int32_t)(hi - lo);
+            const uint64_t *rec = a.stream + offsets[e];
+            uint64_t hdr = rec[0], first = rec[1];
+            int64_t off = offsets[max(e - 1, 0)];
+            int32_t j1 = pbeg ? pbeg[e + 1] : 0, j0 = pbeg ? pbeg[e] : 0;
+            auto const advance = [&]() {
+                rec = a.stream + off;
+                hdr = rec[0];
+                first = rec[1];
+                off = offsets[max(e - 2, 0)];
+                j1 = j0;
+                j0 = pbeg ? pbeg[max(e - 1, 0)] : 0;
+                --e;
+            };
+            while (e >= 0) {
+                // drifts and quadrupoles in a loop of their own: as cases of the
+                // switch they shared its registers, and an element took 149
+                // instructions for its 13 on the FP64 pipe (one warp per
+                // scheduler, a drift 1,300 -> 1,200 cycles, of which 15 FP64
+                // instructions take 1,140; forward and backward 6.76 -> 6.54 ms)
+                while (true) {
+                    bool const drift = (hdr & 0xFF) == OP_DRIFT;
+                    if (!drift && !is_quadrupole(hdr)) break;
+                    bool const on = e <= last;
+                    if (drift) {
+                        double const L = W(first);
+                        advance();
+                        if (on) reverse_drift(s, l, L);
+                    } else {
+                        double const b1 = W(rec[3]);
+                        int32_t const k0 = j0, k1 = j1;
+                        advance();
+                        reverse_quadrupole(s, l, b1, a, k0, k1, on);
+                    }
+                    if (e < 0) break;
+                }
+                if (e < 0) break;
+                const uint64_t *const now = rec;
+                uint64_t const now_hdr = hdr;
+                int32_t const k0 = j0, k1 = j1;
+                bool const on = e <= last;
+                advance();
+                reverse_elem<BB6D>(s, l, now, now_hdr, a, k0, k1, on);
+            }
         }
     }
     if (part) {

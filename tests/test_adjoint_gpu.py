@@ -104,6 +104,39 @@ def test_adjoint_matches_dual_numbers(case, reconstruct):
     assert np.max(np.abs(gp - gp_d) / np.abs(gp_d)) < 1e-8, (gp, gp_d)
 
 
+@pytest.mark.parametrize("order", ["d", "q", "b", "dq", "qd", "bq", "qb", "db", "cd", "qc", "sqd",
+                                   "dqs", "cqqdbdsqc"])
+def test_walk_over_short_lattices(order):
+    """Drifts (d) and quadrupoles (q) at the start, at the end and next to
+    other elements (c cavity, b aperture, s sextupole), particles lost at
+    different elements, against dual numbers (the tolerances of the rings)."""
+    from sixtracklib_gb300.beam_elements import Elements
+
+    e, params = Elements(), []
+    for i, o in enumerate(order):
+        if o == "d":
+            e.Drift(length=1.5)
+        elif o == "c":
+            e.Cavity(voltage=3e6, frequency=4e8, lag=170.0)
+        elif o == "b":
+            e.LimitRect(min_x=-0.015, max_x=0.015, min_y=-0.02, max_y=0.02)
+        else:
+            e.Multipole(knl=[0.0, 0.02] if o == "q" else [0.0, 0.01, 0.3])
+            params.append((i, "knl", 1))
+    if not params:
+        e.Multipole(knl=[0.0, 0.01])
+        params = [(len(order), "knl", 1)]
+    T, n = 4, 130
+    blk = _beam(n, seed=4)
+    w = np.random.default_rng(3).normal(size=(6, n)) / SIGMA[:, None]
+    gc_d, gp_d, vals_d, st_d = _dual_grads(e, params, blk, T, w)
+    gc, gp, vals, st = _gpu_grads(e, params, blk, T, w, every=3)
+    assert np.array_equal(st, st_d)
+    np.testing.assert_allclose(vals, vals_d, rtol=1e-12, atol=1e-18)
+    assert np.all(_rel_rows(gc, gc_d) < 1e-9), _rel_rows(gc, gc_d)
+    assert np.max(np.abs(gp - gp_d) / np.abs(gp_d)) < 1e-8, (gp, gp_d)
+
+
 @pytest.mark.parametrize("p0c", [7e12, 20e9])
 def test_field_kick_adjoints_match_dual_numbers(p0c):
     """RF multipole, 4D beam-beam (round and elliptic), coasting, q-Gaussian
