@@ -467,7 +467,8 @@ void st_Particles_calculate_difference(const st_Particles *lhs, const st_Particl
  * and the reference's TOML forms ("[cuda]\n track_threads_per_block = N",
  * "cuda.threads_per_block = N").  Block sizes are multiples of 32 up to
  * 1024, as in the reference; the tracking kernel (track_threads_per_block,
- * else threads_per_block) runs with at most 256 threads per block. */
+ * else threads_per_block) runs with at most 256 threads per block, and
+ * without either with 32, 64 or 128 by the number of particles. */
 st_TrackJob *st_TrackJob_create(const char *arch, const char *config_str);
 st_TrackJob *st_TrackJob_new(const char *arch, st_Buffer *particles_buffer,
                              st_Buffer *beam_elements_buffer, const char *config_str);
@@ -778,8 +779,8 @@ void st_TrackJobNew_set_collect_flags(st_TrackJobBaseNew *job, uint16_t flags);
 bool st_TrackJobNew_is_collecting_particles(const st_TrackJobBaseNew *job);
 void st_TrackJobNew_enable_collect_particles(st_TrackJobBaseNew *job);
 void st_TrackJobNew_disable_collect_particles(st_TrackJobBaseNew *job);
-/* cuda/track_job.h: the tracking kernel's block size as it runs, and the
- * configured threads_per_block. */
+/* cuda/track_job.h: the tracking kernel's largest block size (the one it runs
+ * with where it is configured), and the configured threads_per_block. */
 uint64_t st_CudaTrackJob_default_track_threads_per_block(const st_CudaTrackJob *job);
 uint64_t st_CudaTrackJob_default_threads_per_block(const st_CudaTrackJob *job);
 
