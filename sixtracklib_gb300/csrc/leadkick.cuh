@@ -218,14 +218,25 @@ STG_HD bool lead_in_range(double x, double y, const uint64_t *blk)
     return ax < lim && ay < lim && (ax >= 0x3D700000u || ay >= 0x3D700000u);
 }
 
+// Whether y is zero or split() keeps all of its bits (2^-66 and above).  The
+// corrections of the exact policy are proportional to y, and with momenta of
+// y's size their last bits count: below, the pair's truncation (2^-24 of y, from
+// 2^-90 down all of it) is outside the bound on them.
+STG_HD bool lead_y_whole(double y)
+{
+    uint64_t const a = bits_of(y) << 1;
+    return a == 0u || a >= 957ull << 53;
+}
+
 STG_HD float lead_error(const LeadTerms &t, uint64_t k)
 {
     return fmul(fadd(fabs_(t.x.h), fabs_(t.y.h)), ffma(high_f(k), t.s.h, low_f(k)));
 }
 
 // u_1 = RN(b_1 + Re(z bracket)) of the exact policy, the corrections v_1 y
-// and v_1 x, v_1 = Im(z bracket), and the bound on v_1 per coordinate.
-// Returns whether u_1 is decided.
+// and v_1 x, v_1 = Im(z bracket), and the bounds on these: 0 only where y is,
+// so that a correction lost below the floats' range is not taken for a known
+// zero.  Returns whether u_1 is decided and the bounds hold.
 STG_HD bool lead_exact(double x, double y, const uint64_t *bal, int order, double *u1,
                        FPair *e1, FPair *e2, float *bound)
 {
@@ -242,9 +253,10 @@ STG_HD bool lead_exact(double x, double y, const uint64_t *bal, int order, doubl
     *e1 = mul(v, t.y);
     *e2 = mul(v, t.x);
     float const d = fmul(fabs_(t.y.h), ffma(high_f(blk[2]), t.s.h, low_f(blk[2])));
-    bound[0] = fmul(fabs_(t.y.h), d);
-    bound[1] = fmul(fabs_(t.x.h), d);
-    return ok;
+    float const least = t.y.h == 0.0f ? 0.0f : 0x1p-149f;
+    bound[0] = ffma(fabs_(t.y.h), d, least);
+    bound[1] = ffma(fabs_(t.x.h), d, least);
+    return ok && lead_y_whole(y);
 }
 
 // RN(k + e), e known to +-d, formed on k's significand; false where the
@@ -280,7 +292,9 @@ STG_HD bool lead_fast(double x, double y, const uint64_t *bal, int order, double
     bool const oka = nearest(FPair{fmul(a.h, scale2), fmul(a.l, scale2)}, d, &ia);
     bool const okb = nearest(FPair{fmul(b.h, scale), fmul(b.l, scale)}, d, &ib);
     *c1 = from_bits(bal[2] + (uint64_t)(ia - ib));
-    double_bounds(mul(t.s, t.g2), fmul(t.s.h, ffma(high_f(blk[2]), t.s.h, low_f(blk[2]))), &w[0],
+    // (the bound never 0, as above)
+    double_bounds(mul(t.s, t.g2),
+                  ffma(t.s.h, ffma(high_f(blk[2]), t.s.h, low_f(blk[2])), 0x1p-149f), &w[0],
                   &w[1]);
     return oka && okb;
 }

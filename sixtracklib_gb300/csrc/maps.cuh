@@ -411,7 +411,7 @@ __device__ __forceinline__ bool lead_kick(PState &p, const uint64_t *bal, int or
 {
     double const x = p.x, y = p.y, chi = p.chi;
     if (!__all_sync(__activemask(), lead_in_range(x, y, bal + 2 * order + 2) &&
-                                        (FAST || is_one(chi))))
+                                        (FAST || (is_one(chi) && lead_y_whole(y)))))
         return false;
     if (FAST) {
         double c1, w[2];

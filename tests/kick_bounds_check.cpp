@@ -1,0 +1,108 @@
+// Checks the kicks of leadkick.cuh on the CPU over the whole range of
+// coordinates and momenta that they accept.  argv: what, samples, seed.
+// Prints "<samples> <undecided> <different>".
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <random>
+
+#include "leadkick.cuh"
+
+using namespace stg;
+
+static std::mt19937_64 gen;
+
+static double uniform() { return (double)(gen() >> 11) * 0x1p-53; }
+static double between(double a, double b) { return a + (b - a) * uniform(); }
+static double sign() { return gen() & 1 ? 1.0 : -1.0; }
+static double normal()
+{
+    return std::sqrt(-2.0 * std::log(uniform() + 0x1p-60)) * std::cos(6.283185307179586 * uniform());
+}
+// of either sign, its logarithm to base 10 uniform
+static double decades(double lo, double hi) { return sign() * std::pow(10.0, between(lo, hi)); }
+static double plus(double v) { return v == 0.0 ? 0.0 : v; }
+
+// One coordinate or both within [1e-12, 8e-3] m, the other down to 1e-40 m or
+// zero; a momentum of the kick's own size, of a beam's, or zero.  Quadrupoles
+// and errors of any strength that gives a lead block.
+static void lead(bool fast, long n, long *undecided, long *different)
+{
+    for (long el = 0; el < n / 100;) {
+        int const order = (fast ? 3 : 2) + (int)(gen() % 9);
+        uint64_t bal[64] = {};
+        double const b1 = decades(-12, 2.9), ratio = std::fabs(decades(-8, 1));
+        bal[2] = bits_of(b1);
+        double scale = std::fabs(b1) * ratio;
+        for (int k = 2; k <= order; ++k) bal[2 * k] = bits_of(normal() * scale), scale *= 0.3;
+        if (!lead_block(bal, order, bal + 2 * order + 2)) continue;
+        ++el;
+        for (int l = 0; l < 100; ++l) {
+            double x = decades(-12, -2.1), y = decades(l & 1 ? -40 : -12, -2.1);
+            if (l % 25 == 0) y = l % 50 ? 0.0 : -0.0;
+            if (l % 4 == 2) std::swap(x, y);
+            double rx, ry;  // the kick: px -= rx, py += ry
+            if (fast) {
+                double const r = x + x, s = std::fma(x, x, y * y);
+                double c1 = from_bits(bal[2 * order]);
+                double c0 = std::fma(r, c1, from_bits(bal[2 * order - 2]));
+                for (int j = order - 2; j >= 1; --j) {
+                    double const cj = std::fma(r, c0, std::fma(-s, c1, from_bits(bal[2 * j])));
+                    c1 = c0;
+                    c0 = cj;
+                }
+                rx = std::fma(x, c0, std::fma(-s, c1, from_bits(bal[0])));
+                ry = y * c0;
+            } else {
+                double u = from_bits(bal[2 * order]), v = 0.0;
+                for (int k = order - 1; k >= 0; --k) {
+                    double const zr = u * x - v * y, zi = u * y + v * x;
+                    u = from_bits(bal[2 * k]) + zr;
+                    v = from_bits(bal[2 * k + 1]) + zi;
+                }
+                rx = u;
+                ry = v;
+            }
+            int const m = (int)(gen() % 4);
+            double const px = m == 0 ? 1e-5 * normal() : m == 1 ? 0.0 : rx * decades(-3, 3);
+            double const py = m == 0 ? 1e-5 * normal() : m == 1 ? 0.0 : ry * decades(-3, 3);
+            double a, b, c, d;
+            bool ok = lead_in_range(x, y, bal + 2 * order + 2);
+            if (fast) {
+                double u1, w[2];
+                ok = ok && lead_fast(x, y, bal, order, &u1, w);
+                a = px - std::fma(x, u1, -w[0]), b = px - std::fma(x, u1, -w[1]);
+                c = d = py + y * u1;
+            } else {
+                double u1, s1, s2, b1[2], b2[2];
+                FPair e1, e2;
+                float dd[2];
+                ok = ok && lead_exact(x, y, bal, order, &u1, &e1, &e2, dd);
+                double const kx = u1 * x, ky = u1 * y;
+                FPair const m1{-e1.h, -e1.l};
+                double_bounds(m1, dd[0], &b1[0], &b1[1]);
+                double_bounds(e2, dd[1], &b2[0], &b2[1]);
+                a = px - plus(kx + b1[0]), b = px - plus(kx + b1[1]);
+                c = py + plus(ky + b2[0]), d = py + plus(ky + b2[1]);
+                if (nearest_sum(kx, m1, dd[0], &s1)) a = b = px - s1;
+                if (nearest_sum(ky, e2, dd[1], &s2)) c = d = py + s2;
+            }
+            if (!ok || bits_of(a) != bits_of(b) || bits_of(c) != bits_of(d))
+                ++*undecided;
+            else if (bits_of(a) != bits_of(px - rx) || bits_of(c) != bits_of(py + ry))
+                ++*different;
+        }
+    }
+}
+
+int main(int argc, char **argv)
+{
+    if (argc < 4) return 2;
+    long const n = atol(argv[2]);
+    gen.seed((uint64_t)atol(argv[3]));
+    long undecided = 0, different = 0;
+    lead(!strcmp(argv[1], "lead fast"), n, &undecided, &different);
+    printf("%ld %ld %ld\n", n, undecided, different);
+    return 0;
+}

@@ -1,0 +1,35 @@
+"""The kicks evaluated in pairs of floats (csrc/leadkick.cuh), on the CPU, over
+the whole range of coordinates and momenta that they accept: what they decide
+has the FP64 sequence's bits."""
+
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "sixtracklib_gb300", "csrc")
+
+
+@pytest.fixture(scope="module")
+def check(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("kick_bounds") / "check")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-x", "c++", "-I" + CSRC,
+                    os.path.join(HERE, "kick_bounds_check.cpp"), "-o", exe], check=True)
+
+    def run(what, n, seed):
+        out = subprocess.run([exe, what, str(n), str(seed)], check=True, capture_output=True,
+                             text=True).stdout
+        return [int(v) for v in out.split()]
+
+    return run
+
+
+@pytest.mark.parametrize("what", ["lead exact", "lead fast"])
+def test_lead_kick_at_small_coordinates(check, what):
+    """One coordinate down to 1e-40 m, momenta of the kick's own size: there the
+    last bits of the corrections to u_1 x and u_1 y show."""
+    n, undecided, different = check(what, 1_000_000, 17)
+    print(f"{what}: {undecided} of {n} left to the FP64 sequence")
+    assert different == 0
+    assert undecided < n
