@@ -386,6 +386,8 @@ STG_HD bool sc_pair_kick(double x, double y, FPair k, double zeta, double inv_rv
     FPair const K = mul(mul(k, pair_of(blk[0])), exp_pair(az));
     if (round) {
         FPair const r2 = mul_add_mul(X, X, Y, Y);
+        // within 1e-10 m of the axis the field is another, sqrt(r2) / sigma
+        if (r2.h < 1.0001e-20f) return false;
         FPair u = neg(mul(r2, pair_of(blk[3])));
         if (u.h < -80.0f) u = FPair{-80.0f, 0.0f};
         FPair const e = exp_pair(u), one = two_sum(1.0f, -e.h);

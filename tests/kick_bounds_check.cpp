@@ -1,4 +1,4 @@
-// Checks the kicks of leadkick.cuh on the CPU over the whole range of
+// Checks the kicks of leadkick.cuh and sckick.cuh on the CPU over the whole range of
 // coordinates and momenta that they accept.  argv: what, samples, seed.
 // Prints "<samples> <undecided> <different>".
 #include <cmath>
@@ -7,7 +7,7 @@
 #include <cstring>
 #include <random>
 
-#include "leadkick.cuh"
+#include "sckick.cuh"
 
 using namespace stg;
 
@@ -96,13 +96,75 @@ static void lead(bool fast, long n, long *undecided, long *different)
     }
 }
 
+// Round space charge of a Gaussian beam: the field's two forms, the one within
+// 1e-10 m of the axis included.  A kick outside its bounds counts as different
+// whether its momenta are decided or not.
+struct Round {
+    double sigma, sb, line;
+    uint64_t blk[kScPairWords];
+    long double factor;
+
+    bool make(double s, double bunch)
+    {
+        constexpr long double two_pi_eps0 = 2.0L * 3.14159265358979323846L * 8.854187817620e-12L;
+        sigma = s;
+        sb = 1.0 / (std::sqrt(2.0) * bunch);
+        line = 0.1 * 1e11 * sb / std::sqrt(3.14159265358979323846);
+        factor = line / two_pi_eps0;
+        return sc_pair_block(line, sb, true, s, s, s, blk);
+    }
+
+    void one(double x, double y, double zeta, double irv, double k0, double room, long *undecided,
+             long *different) const
+    {
+        long double const z = (long double)zeta * irv, r2 = (long double)x * x + (long double)y * y;
+        long double const K = k0 * factor * expl(-(long double)sb * sb * z * z);
+        long double const t = r2 < 1e-20L ? sqrtl(r2) / sigma
+                                          : -expm1l(-0.5L * r2 / ((long double)sigma * sigma)) / r2;
+        long double const ex = K * t * x, ey = K * t * y;
+        // momenta from the smallest that may be decided up
+        double const top = (double)(k0 * factor) * 0.46 / sigma * 16500.0;
+        double const px = sign() * top * room, py = sign() * top * room * between(1, 2);
+        FPair const k = sc_factor(k0);
+        double kx[2], ky[2];
+        if (!sc_small(k, px, py, blk) ||
+            !sc_pair_kick(x, y, k, zeta, irv, blk, true, false, kx, ky)) {
+            ++*undecided;
+            return;
+        }
+        bool const in = std::fmin(kx[0], kx[1]) <= ex && ex <= std::fmax(kx[0], kx[1]) &&
+                        std::fmin(ky[0], ky[1]) <= ey && ey <= std::fmax(ky[0], ky[1]);
+        bool const same = px + kx[0] == px + kx[1] && py + ky[0] == py + ky[1];
+        if (!in || (same && (px + kx[0] != px + (double)ex || py + ky[0] != py + (double)ey)))
+            ++*different;
+        else if (!same)
+            ++*undecided;
+    }
+};
+
+static void near_axis(long n, long *undecided, long *different)
+{
+    for (long i = 0; i < n;) {
+        Round b;
+        if (!b.make(std::fabs(decades(-6, -3)), 0.1)) continue;
+        for (int l = 0; l < 100; ++l, ++i) {
+            double const x = decades(-13, -8), y = decades(-13, -8);
+            b.one(x, y, 0.05 * normal(), 1.0 + 1e-6 * normal(), 3.9e-40 * between(1, 2),
+                  std::fabs(decades(0, 4)), undecided, different);
+        }
+    }
+}
+
 int main(int argc, char **argv)
 {
     if (argc < 4) return 2;
     long const n = atol(argv[2]);
     gen.seed((uint64_t)atol(argv[3]));
     long undecided = 0, different = 0;
-    lead(!strcmp(argv[1], "lead fast"), n, &undecided, &different);
+    if (!strcmp(argv[1], "near axis"))
+        near_axis(n, &undecided, &different);
+    else
+        lead(!strcmp(argv[1], "lead fast"), n, &undecided, &different);
     printf("%ld %ld %ld\n", n, undecided, different);
     return 0;
 }

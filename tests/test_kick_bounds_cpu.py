@@ -1,6 +1,6 @@
-"""The kicks evaluated in pairs of floats (csrc/leadkick.cuh), on the CPU, over
-the whole range of coordinates and momenta that they accept: what they decide
-has the FP64 sequence's bits."""
+"""The kicks evaluated in pairs of floats (csrc/leadkick.cuh,
+csrc/sckick.cuh), on the CPU, over the whole range of coordinates and momenta
+that they accept: what they decide has the FP64 sequence's bits."""
 
 import os
 import subprocess
@@ -31,5 +31,14 @@ def test_lead_kick_at_small_coordinates(check, what):
     last bits of the corrections to u_1 x and u_1 y show."""
     n, undecided, different = check(what, 1_000_000, 17)
     print(f"{what}: {undecided} of {n} left to the FP64 sequence")
+    assert different == 0
+    assert undecided < n
+
+
+def test_round_space_charge_near_the_axis(check):
+    """Beams of 1 um to 1 mm, particles from 1e-13 to 1e-8 m: the field has
+    another form within 1e-10 m of the axis."""
+    n, undecided, different = check("near axis", 1_000_000, 19)
+    print(f"{undecided} of {n} left to the FP64 evaluation")
     assert different == 0
     assert undecided < n
