@@ -143,8 +143,10 @@ STG_HD FPair div(FPair a, FPair b)
     return renorm(q, fmul(rem, r));
 }
 
-// e^x for a pair -80 <= x <= 0: x = n ln2 / 32 + r.  To 2^-42 relative down to
-// x = -60, where the low part leaves the normal range.
+// e^x for a pair -80 <= x <= 0 by P. T. P. Tang's table-driven method (ACM
+// TOMS 15 (1989) 144): x = n ln2 / 32 + r.  With u = 2^-24, to 24 u^2 relative
+// and 5 u |x.l| for the sums that the low part passes through; below x = -60
+// the result's low part leaves the normal range.
 STG_HD FPair exp_pair(FPair x)
 {
     constexpr float kMagic = 12582912.0f;  // 1.5 2^23
@@ -384,6 +386,18 @@ STG_HD bool sc_pair_kick(double x, double y, FPair k, double zeta, double inv_rv
     FPair const az = neg(mul(mul(z, z), pair_of(blk[2])));
     if (az.h < -60.0f) return false;
     FPair const K = mul(mul(k, pair_of(blk[0])), exp_pair(az));
+    // The bound.  With u = 2^-24 the low part of a split number is at most 2 u
+    // of it and mul() of pairs with low parts a and b (in units of u) errs by
+    // ab + 3 + 3a + 2b or so (u^2): zeta / rvv by 14 u^2, az by 97 u^2 with a
+    // low part of 13 u, whose sums in exp_pair add 65 u^2 |az| to its own 24 u^2.
+    // K is known to (162 |az| + 46) u^2; the round field adds 38 (its exponent),
+    // 26 (difference and quotient) and 10 (times X), the elliptic one 67 of
+    // |w| or less: below (162 |az| + 120) u^2, of which the FP64 evaluation's
+    // own roundings and those of double_bounds take less than one.  Far out K or
+    // the kick may leave the floats' range: never a bound of 0, which would
+    // stand for a known kick of 0 (below 2^-75 double_bounds allows 2^-100).
+    constexpr float kLeast = 0x1p-149f;
+    float const rel = ffma(-az.h, 0x1.6p-41f, 0x1.2p-41f);  // (176 |az| + 144) u^2
     if (round) {
         FPair const r2 = mul_add_mul(X, X, Y, Y);
         // within 1e-10 m of the axis the field is another, sqrt(r2) / sigma
@@ -392,10 +406,9 @@ STG_HD bool sc_pair_kick(double x, double y, FPair k, double zeta, double inv_rv
         if (u.h < -80.0f) u = FPair{-80.0f, 0.0f};
         FPair const e = exp_pair(u), one = two_sum(1.0f, -e.h);
         FPair const g = mul(K, div(renorm(one.h, fsub(one.l, e.l)), r2));
-        // e and the quotients to 2^-42 or better
-        float const d = fmul(fmul(K.h, frcp(r2.h)), 0x1p-41f);
-        double_bounds(mul(X, g), fmul(fabs_(X.h), d), &kx[0], &kx[1]);
-        double_bounds(mul(Y, g), fmul(fabs_(Y.h), d), &ky[0], &ky[1]);
+        float const d = fmul(fmul(K.h, frcp(r2.h)), rel);
+        double_bounds(mul(X, g), ffma(fabs_(X.h), d, kLeast), &kx[0], &kx[1]);
+        double_bounds(mul(Y, g), ffma(fabs_(Y.h), d, kLeast), &ky[0], &ky[1]);
         return true;
     }
     FPair const ax{fabs_(X.h), X.h < 0.0f ? -X.l : X.l}, ay{fabs_(Y.h), Y.h < 0.0f ? -Y.l : Y.l};
@@ -411,8 +424,8 @@ STG_HD bool sc_pair_kick(double x, double y, FPair k, double zeta, double inv_rv
     if (arg.h < -80.0f) arg = FPair{-80.0f, 0.0f};
     FPair const e = exp_pair(arg);
     FPair const fu = mul(K, add(w1i, neg(mul(w2i, e)))), fv = mul(K, add(w1r, neg(mul(w2r, e))));
-    float const d = fmul(fmul(K.h, fadd(fadd(w1r.h, w1i.h), fmul(e.h, fadd(w2r.h, w2i.h)))),
-                         0x1p-41f);
+    float const d = ffma(fmul(K.h, fadd(fadd(w1r.h, w1i.h), fmul(e.h, fadd(w2r.h, w2i.h)))),
+                         rel, kLeast);
     FPair fx = wide_x ? fu : fv, fy = wide_x ? fv : fu;
     if (X.h < 0.0f) fx = neg(fx);
     if (Y.h < 0.0f) fy = neg(fy);
@@ -429,6 +442,8 @@ inline bool sc_pair_block(double line, double sqrt_beta, bool round, double sigm
 {
     constexpr double pi = 3.14159265358979323846, eps0 = 8.854187817620e-12;
     constexpr double sqrt_pi = 1.77245385090551602730;
+    // a round field of 2^30 K, so that K keeps its low part for kicks of 2^-75
+    if (round && !(sigma > 0x1p-30)) return false;
     double const su = sx > sy ? sx : sy, sv = sx > sy ? sy : sx;
     double const S = std::sqrt(2.0 * (su * su - sv * sv));
     double const factor = std::ldexp(

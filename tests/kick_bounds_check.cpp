@@ -96,39 +96,83 @@ static void lead(bool fast, long n, long *undecided, long *different)
     }
 }
 
-// Round space charge of a Gaussian beam: the field's two forms, the one within
-// 1e-10 m of the axis included.  A kick outside its bounds counts as different
-// whether its momenta are decided or not.
-struct Round {
-    double sigma, sb, line;
+// The Faddeeva function of the CERN algorithm in long double (x, y > 0).
+static void cerrf(double x, double y, long double *wr, long double *wi)
+{
+    bool const inner = x < 5.33 && y < 4.29;
+    double const q = inner ? (1.0 - y / 4.29) * std::sqrt(1.0 - (x / 5.33) * (x / 5.33)) : 0.0;
+    int const nc = inner ? 7 + (int)(23.0 * q) : 1, nu = inner ? 10 + (int)(21.0 * q) : 9;
+    long double const g = 1.6 * q, u = y + g, v = x;
+    long double q1r = 1, q1i = 0, q2r = 0, q2i = 0, ar = 0, ai = 0;
+    for (int n = nu; n > 0; --n) {
+        if (n <= nc) ar = ar * g + q1r, ai = ai * g + q1i;
+        long double const qr = u * q1r - v * q1i + 0.5L * n * q2r;
+        long double const qi = u * q1i + v * q1r + 0.5L * n * q2i;
+        q2r = q1r, q2i = q1i, q1r = qr, q1i = qi;
+    }
+    long double const c = 0.5L * 1.12837916709551L / (q1r * q1r + q1i * q1i);
+    *wr = (ar * q1r + ai * q1i) * c;
+    *wi = (ar * q1i - ai * q1r) * c;
+}
+
+// Space charge of a Gaussian beam; of the round field both forms, the one
+// within 1e-10 m of the axis included.  A kick outside its bounds counts as
+// different whether its momenta are decided or not.
+struct Beam {
+    double sx, sy, sb, line;
     uint64_t blk[kScPairWords];
     long double factor;
 
-    bool make(double s, double bunch)
+    bool make(double x, double y, double bunch)
     {
-        constexpr long double two_pi_eps0 = 2.0L * 3.14159265358979323846L * 8.854187817620e-12L;
-        sigma = s;
+        constexpr long double pi = 3.14159265358979323846L, eps0 = 8.854187817620e-12L;
+        sx = x;
+        sy = y;
         sb = 1.0 / (std::sqrt(2.0) * bunch);
         line = 0.1 * 1e11 * sb / std::sqrt(3.14159265358979323846);
-        factor = line / two_pi_eps0;
-        return sc_pair_block(line, sb, true, s, s, s, blk);
+        double const su = std::fmax(sx, sy), sv = std::fmin(sx, sy);
+        factor = line / (sx == sy ? 2 * pi * eps0
+                                  : 2 * eps0 * sqrtl(pi * 2.0L * (su * su - sv * sv)));
+        return sc_pair_block(line, sb, sx == sy, 0.5 * (sx + sy), sx, sy, blk);
+    }
+
+    void field(double x, double y, long double *ex, long double *ey) const
+    {
+        if (sx == sy) {
+            long double const r2 = (long double)x * x + (long double)y * y, s = sx;
+            long double const t = r2 < 1e-20L ? sqrtl(r2) / s : -expm1l(-0.5L * r2 / (s * s)) / r2;
+            *ex = t * x, *ey = t * y;
+            return;
+        }
+        bool const wide = sx > sy;
+        double const su = std::fmax(sx, sy), sv = std::fmin(sx, sy);
+        double const S = std::sqrt(2.0 * (su * su - sv * sv));
+        double const u = std::fabs(wide ? x : y), v = std::fabs(wide ? y : x);
+        long double a, b, c, d;
+        cerrf(u / S, v / S, &a, &b);
+        cerrf(sv / su * u / S, su / sv * v / S, &c, &d);
+        long double const e = expl(-0.5L * ((long double)u * u / ((long double)su * su) +
+                                            (long double)v * v / ((long double)sv * sv)));
+        long double const fu = b - d * e, fv = a - c * e;
+        *ex = std::copysign(1.0, x) * (wide ? fu : fv);
+        *ey = std::copysign(1.0, y) * (wide ? fv : fu);
     }
 
     void one(double x, double y, double zeta, double irv, double k0, double room, long *undecided,
              long *different) const
     {
-        long double const z = (long double)zeta * irv, r2 = (long double)x * x + (long double)y * y;
+        long double const z = (long double)zeta * irv;
         long double const K = k0 * factor * expl(-(long double)sb * sb * z * z);
-        long double const t = r2 < 1e-20L ? sqrtl(r2) / sigma
-                                          : -expm1l(-0.5L * r2 / ((long double)sigma * sigma)) / r2;
-        long double const ex = K * t * x, ey = K * t * y;
+        long double ex, ey;
+        field(x, y, &ex, &ey);
+        ex *= K, ey *= K;
         // momenta from the smallest that may be decided up
-        double const top = (double)(k0 * factor) * 0.46 / sigma * 16500.0;
+        double const top = (double)(k0 * factor) * (sx == sy ? 0.46 / sx : 1.0) * 16500.0;
         double const px = sign() * top * room, py = sign() * top * room * between(1, 2);
         FPair const k = sc_factor(k0);
         double kx[2], ky[2];
         if (!sc_small(k, px, py, blk) ||
-            !sc_pair_kick(x, y, k, zeta, irv, blk, true, false, kx, ky)) {
+            !sc_pair_kick(x, y, k, zeta, irv, blk, sx == sy, sx > sy, kx, ky)) {
             ++*undecided;
             return;
         }
@@ -145,12 +189,31 @@ struct Round {
 static void near_axis(long n, long *undecided, long *different)
 {
     for (long i = 0; i < n;) {
-        Round b;
-        if (!b.make(std::fabs(decades(-6, -3)), 0.1)) continue;
+        double const sigma = std::fabs(decades(-6, -3));
+        Beam b;
+        if (!b.make(sigma, sigma, 0.1)) continue;
         for (int l = 0; l < 100; ++l, ++i) {
             double const x = decades(-13, -8), y = decades(-13, -8);
             b.one(x, y, 0.05 * normal(), 1.0 + 1e-6 * normal(), 3.9e-40 * between(1, 2),
                   std::fabs(decades(0, 4)), undecided, different);
+        }
+    }
+}
+
+// The longitudinal exponent over its whole range, particles within four sigma.
+static void tails(bool round, long n, long *undecided, long *different)
+{
+    for (long i = 0; i < n;) {
+        double const sx = std::fabs(decades(-8, -2));
+        Beam b;
+        if (!b.make(sx, round ? sx : sx * std::fabs(decades(-1.5, 1.5)),
+                    std::fabs(decades(-3, -0.5))))
+            continue;
+        for (int l = 0; l < 100; ++l, ++i) {
+            double const x = 4 * b.sx * between(-1, 1), y = 4 * b.sy * between(-1, 1);
+            b.one(x, y, sign() * std::sqrt(61.0 * uniform()) / b.sb, 1.0 + 1e-6 * normal(),
+                  3.9e-40 * std::fabs(decades(-3, 3)), std::fabs(decades(0, 4)), undecided,
+                  different);
         }
     }
 }
@@ -163,6 +226,8 @@ int main(int argc, char **argv)
     long undecided = 0, different = 0;
     if (!strcmp(argv[1], "near axis"))
         near_axis(n, &undecided, &different);
+    else if (!strncmp(argv[1], "tails", 5))
+        tails(!strcmp(argv[1], "tails round"), n, &undecided, &different);
     else
         lead(!strcmp(argv[1], "lead fast"), n, &undecided, &different);
     printf("%ld %ld %ld\n", n, undecided, different);

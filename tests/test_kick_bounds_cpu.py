@@ -42,3 +42,13 @@ def test_round_space_charge_near_the_axis(check):
     print(f"{undecided} of {n} left to the FP64 evaluation")
     assert different == 0
     assert undecided < n
+
+
+@pytest.mark.parametrize("beam", ["round", "elliptic"])
+def test_space_charge_bounds_over_the_bunch(check, beam):
+    """The longitudinal exponent over its whole range, beams of 10 nm to 1 cm
+    and bunches of 1 mm to 0.3 m: the bounds hold every kick."""
+    n, undecided, different = check(f"tails {beam}", 500_000, 31)
+    print(f"{beam}: {undecided} of {n} left to the FP64 evaluation")
+    assert different == 0
+    assert undecided < n
