@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "common.h"
+#include "column_copy.h"
 #include "kernel_api.h"
 #include "device_guard.h"
 #include "lattice.h"
@@ -996,41 +997,32 @@ bool in_pinned(const st_TrackJob *j, const st_Particles *p, int64_t cnt)
     return true;
 }
 
-// The columns of p (cnt particles) to or from rows of `pitch` words on the
-// device, straight between the two memories; a null stream copies as
-// cudaMemcpy does.  Columns at one distance, as the buffers lay them out, go in
-// one copy: the host's work for each of 42 copies bounded a small set (push
-// and collect of 1,000 particles from Python 257 -> 61 us with the columns
-// read in one piece there), a staging block with its pages to fault in and its
-// second pass over memory a large one (34 MB of element-by-element output 6.8
-// -> 0.19 ms).
-bool copy_columns(st_Particles *p, int64_t cnt, uint64_t *d, int64_t pitch, bool to_device,
-                  cudaStream_t s, const char *what)
-{
-    if (cnt <= 0) return true;
-    size_t const width = (size_t)cnt * 8, dev = (size_t)pitch * 8;
-    cudaMemcpyKind const kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
-    uintptr_t const first = (uintptr_t)column(p, 0);
-    size_t const apart = (uintptr_t)column(p, 1) - first;
-    constexpr size_t kMaxPitch = 0x7fffffff;  // of a pitched copy
-    bool even = (uintptr_t)column(p, 1) > first && apart >= width;
-    for (int c = 2; c < 21; ++c) even = even && (uintptr_t)column(p, c) == first + c * apart;
-    bool const one = even && apart == width && dev == width;
-    bool const pitched = even && apart <= kMaxPitch && dev <= kMaxPitch;
-    size_t const bytes = one ? 21 * width : width;
-    for (int c = 0; c < (one || pitched ? 1 : 21); ++c) {
-        void *const host = column(p, c), *const there = d + (size_t)c * pitch;
-        void *const to = to_device ? there : host, *const from = to_device ? host : there;
-        size_t const tp = to_device ? dev : apart, fp = to_device ? apart : dev;
-        cudaError_t e;
-        if (!one && pitched)
-            e = s ? cudaMemcpy2DAsync(to, tp, from, fp, width, 21, kind, s)
-                  : cudaMemcpy2D(to, tp, from, fp, width, 21, kind);
-        else
-            e = s ? cudaMemcpyAsync(to, from, bytes, kind, s) : cudaMemcpy(to, from, bytes, kind);
-        if (!cuda_ok(e, what)) return false;
+// The runtime's copies for column_copy.h, on `stream`: null copies as
+// cudaMemcpy does.
+struct RuntimeCopies {
+    cudaMemcpyKind kind;
+    cudaStream_t stream;
+    const char *what;
+    bool copy(void *to, const void *from, size_t bytes)
+    {
+        return cuda_ok(stream ? cudaMemcpyAsync(to, from, bytes, kind, stream)
+                              : cudaMemcpy(to, from, bytes, kind),
+                       what);
     }
-    return true;
+    bool copy2d(void *to, size_t tp, const void *from, size_t fp, size_t width, size_t rows)
+    {
+        return cuda_ok(stream ? cudaMemcpy2DAsync(to, tp, from, fp, width, rows, kind, stream)
+                              : cudaMemcpy2D(to, tp, from, fp, width, rows, kind),
+                       what);
+    }
+    bool wait() { return cuda_ok(cudaStreamSynchronize(stream), what); }
+};
+
+ColumnSet column_set(const st_Particles *p, int64_t cnt, uint64_t *d, int64_t pitch)
+{
+    ColumnSet s{{}, cnt, d, pitch};
+    for (int c = 0; c < 21; ++c) s.cols[c] = column(p, c);
+    return s;
 }
 
 // The particle sets between the caller's buffer and the device block: copies
@@ -1038,14 +1030,15 @@ bool copy_columns(st_Particles *p, int64_t cnt, uint64_t *d, int64_t pitch, bool
 bool copy_particles(st_TrackJob *j, bool to_device)
 {
     bool pinned = j->pinned != nullptr;
-    for (size_t k = 0; pinned && k < j->psets.size(); ++k)
-        pinned = in_pinned(j, pset(j, k), j->pset_cnt[k]);
-    cudaStream_t const s = pinned ? j->dev->stream : nullptr;
-    for (size_t k = 0; k < j->psets.size(); ++k)
-        if (!copy_columns(pset(j, k), j->pset_cnt[k], j->d_cols + j->pset_off[k], j->n_total,
-                          to_device, s, "cudaMemcpy(particles)"))
-            return false;
-    return !pinned || cuda_ok(cudaStreamSynchronize(s), "particle copy");
+    std::vector<ColumnSet> sets;
+    for (size_t k = 0; k < j->psets.size(); ++k) {
+        const st_Particles *const p = pset(j, k);
+        pinned = pinned && in_pinned(j, p, j->pset_cnt[k]);
+        sets.push_back(column_set(p, j->pset_cnt[k], j->d_cols + j->pset_off[k], j->n_total));
+    }
+    RuntimeCopies api{to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost,
+                      pinned ? j->dev->stream : nullptr, "cudaMemcpy(particles)"};
+    return copy_sets(api, sets, to_device);
 }
 
 bool upload_particles(st_TrackJob *j) { return copy_particles(j, true); }
@@ -1053,12 +1046,15 @@ bool download_particles(st_TrackJob *j) { return copy_particles(j, false); }
 
 bool transfer_outputs(st_TrackJob *j, bool to_device)
 {
+    std::vector<ColumnSet> sets;
     for (const OutBlock &o : j->outs) {
-        st_Particles *p = st_Particles_buffer_get_particles(j->obuf, o.obj_index);
-        if (!p || !copy_columns(p, o.cap, o.d, o.cap, to_device, nullptr, "cudaMemcpy(output)"))
-            return false;
+        const st_Particles *const p = st_Particles_buffer_get_particles(j->obuf, o.obj_index);
+        if (!p) return false;
+        sets.push_back(column_set(p, o.cap, o.d, o.cap));
     }
-    return true;
+    RuntimeCopies api{to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, nullptr,
+                      "cudaMemcpy(output)"};
+    return copy_sets(api, sets, to_device);
 }
 
 bool compile_job_lattice(st_TrackJob *j)
