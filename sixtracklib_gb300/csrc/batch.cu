@@ -31,6 +31,7 @@
 #include "device_guard.h"
 #include "kernel_api.h"
 #include "lattice_view.h"
+#include "runtime_copies.h"
 
 namespace stg {
 namespace {
@@ -227,13 +228,9 @@ bool build_plan(st_BatchTracker *b, const Shape &sh, const std::vector<uint64_t 
         p.release();
         return false;
     }
-    if (!cuda_ok(cudaMemcpy(p.d_variants, prm.data(), V * sizeof(TrackParams),
-                            cudaMemcpyHostToDevice),
-                 "cudaMemcpy(batch variants)") ||
-        (!items.empty() &&
-         !cuda_ok(cudaMemcpy(p.d_items, items.data(), items.size() * sizeof(BatchItem),
-                             cudaMemcpyHostToDevice),
-                  "cudaMemcpy(batch items)"))) {
+    if (!upload({{p.d_variants, prm.data(), V * sizeof(TrackParams)},
+                 {p.d_items, items.data(), items.size() * sizeof(BatchItem)}},
+                "cudaMemcpy(batch plan)")) {
         p.release();
         return false;
     }

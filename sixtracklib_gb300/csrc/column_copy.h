@@ -1,10 +1,11 @@
-// column_copy.h -- a job's particle columns between host and device memory,
-// written against the few calls of the CUDA runtime that it needs, so that
-// the order of copies and waits is checked on the CPU.
+// column_copy.h -- a job's particle columns between host and device memory, and
+// tables from host to device, written against the few calls of the CUDA runtime
+// that they need, so that the order of copies and waits is checked on the CPU.
 #pragma once
 
 #include <cstddef>
 #include <cstdint>
+#include <initializer_list>
 #include <vector>
 
 namespace stg {
@@ -58,6 +59,22 @@ bool copy_sets(Api &api, const std::vector<ColumnSet> &sets, bool to_device)
 {
     bool ok = true;
     for (const ColumnSet &s : sets) ok = ok && copy_columns(api, s, to_device);
+    return api.wait() && ok;
+}
+
+struct BlockCopy {
+    void *to;
+    const void *from;
+    size_t bytes;
+};
+
+// Blocks of words, and the wait for all of them.
+template <class Api>
+bool copy_blocks(Api &api, std::initializer_list<BlockCopy> blocks)
+{
+    bool ok = true;
+    for (const BlockCopy &b : blocks)
+        ok = ok && (b.bytes == 0 || api.copy(b.to, b.from, b.bytes));
     return api.wait() && ok;
 }
 

@@ -26,11 +26,11 @@
 #include <vector>
 
 #include "common.h"
-#include "column_copy.h"
 #include "kernel_api.h"
 #include "device_guard.h"
 #include "lattice.h"
 #include "leadkick.cuh"
+#include "runtime_copies.h"
 
 extern "C" uint64_t stg_buffer_generation(const st_Buffer *b);
 
@@ -314,18 +314,12 @@ static std::unique_ptr<DevStream> build_stream(const ImageView &img, uint64_t b,
     // out-of-line tables: their device addresses go into the records
     uint64_t const side_base = (uint64_t)(uintptr_t)s->d + side_at;
     for (const auto &f : s->cs.side_fixups) s->cs.words[f.first] = side_base + f.second * 8u;
-    if ((side_bytes > 0 &&
-         !cuda_ok(cudaMemcpy(reinterpret_cast<char *>(s->d) + side_at, s->cs.side.data(),
-                             side_bytes, cudaMemcpyHostToDevice),
-                  "cudaMemcpy(side tables)")) ||
-        !cuda_ok(cudaMemcpy(reinterpret_cast<char *>(s->d) + bytes + sbytes,
-                            s->cs.elem_offset.data(), obytes, cudaMemcpyHostToDevice),
-                 "cudaMemcpy(element offsets)") ||
-        !cuda_ok(cudaMemcpy(s->d, s->cs.words.data(), bytes, cudaMemcpyHostToDevice),
-                 "cudaMemcpy(lattice)") ||
-        !cuda_ok(cudaMemcpy(reinterpret_cast<char *>(s->d) + bytes, s->cs.s_table.data(), sbytes,
-                            cudaMemcpyHostToDevice),
-                 "cudaMemcpy(s table)"))
+    char *const base = reinterpret_cast<char *>(s->d);
+    if (!upload({{base + side_at, s->cs.side.data(), side_bytes},
+                 {base + bytes + sbytes, s->cs.elem_offset.data(), obytes},
+                 {base, s->cs.words.data(), bytes},
+                 {base + bytes, s->cs.s_table.data(), sbytes}},
+                "cudaMemcpy(lattice)"))
         return nullptr;
     // TriCub cell coefficients, computed on the GPU from the node tables
     if (!s->cs.tricub_tables.empty()) {
@@ -804,9 +798,7 @@ st_track_status_t st_DeviceLattice_set_parameters(st_DeviceLattice *L, int64_t n
             aux |= MP_LEAD;
         hdr = (hdr & 0xFFFFFFFFull) | ((uint64_t)aux << 32);
     }
-    if (!cuda_ok(cudaMemcpy(ds.d, ds.cs.words.data(), ds.cs.words.size() * 8,
-                            cudaMemcpyHostToDevice),
-                 "cudaMemcpy(lattice)"))
+    if (!upload({{ds.d, ds.cs.words.data(), ds.cs.words.size() * 8}}, "cudaMemcpy(lattice)"))
         return -1;
     L->lines.clear();  // line streams are rebuilt from the updated image
     return 0;
@@ -996,27 +988,6 @@ bool in_pinned(const st_TrackJob *j, const st_Particles *p, int64_t cnt)
     }
     return true;
 }
-
-// The runtime's copies for column_copy.h, on `stream`: null copies as
-// cudaMemcpy does.
-struct RuntimeCopies {
-    cudaMemcpyKind kind;
-    cudaStream_t stream;
-    const char *what;
-    bool copy(void *to, const void *from, size_t bytes)
-    {
-        return cuda_ok(stream ? cudaMemcpyAsync(to, from, bytes, kind, stream)
-                              : cudaMemcpy(to, from, bytes, kind),
-                       what);
-    }
-    bool copy2d(void *to, size_t tp, const void *from, size_t fp, size_t width, size_t rows)
-    {
-        return cuda_ok(stream ? cudaMemcpy2DAsync(to, tp, from, fp, width, rows, kind, stream)
-                              : cudaMemcpy2D(to, tp, from, fp, width, rows, kind),
-                       what);
-    }
-    bool wait() { return cuda_ok(cudaStreamSynchronize(stream), what); }
-};
 
 ColumnSet column_set(const st_Particles *p, int64_t cnt, uint64_t *d, int64_t pitch)
 {

@@ -43,9 +43,24 @@ struct Fake {
     }
 };
 
+static int blocks(int fail)
+{
+    std::vector<uint64_t> const a(9, 3), b(5, 4);
+    std::vector<uint64_t> dev(14, 0);
+    Fake api{true, fail};
+    bool const done =
+        copy_blocks(api, {{dev.data(), a.data(), 72}, {nullptr, nullptr, 0}, {&dev[9], b.data(), 40}});
+    if (!api.flight.empty()) return puts("copies in flight after the return"), 0;
+    if (done != (fail < 0 || fail >= api.calls)) return puts("a failure was not reported"), 0;
+    for (int i = 0; done && i < 14; ++i)
+        if (dev[i] != (i < 9 ? 3u : 4u)) return printf("word %d\n", i), 0;
+    return puts("ok"), 0;
+}
+
 int main(int argc, char **argv)
 {
     if (argc < 4) return 2;
+    if (!strcmp(argv[1], "blocks")) return blocks(atoi(argv[3]));
     bool const to_device = !strcmp(argv[2], "up");
     int const fail = atoi(argv[3]);
     // two sets in one block on the device; the host's columns back to back, at

@@ -1,4 +1,4 @@
-"""A job's column copies (csrc/column_copy.h) on the CPU, against a runtime
+"""A job's column copies and the upload of tables (csrc/column_copy.h) on the CPU, against a runtime
 whose copies to the device land only when their stream is waited for."""
 
 import os
@@ -31,3 +31,9 @@ def test_columns_have_arrived_on_return(check, layout, direction):
     assert check(layout, direction, -1) == "ok"
     for fail in (0, 1, 30):
         assert check(layout, direction, fail) == "ok"
+
+
+def test_tables_have_arrived_on_return(check):
+    """Several blocks, an empty one among them."""
+    for fail in (-1, 0, 1, 2):
+        assert check("blocks", "up", fail) == "ok"
