@@ -193,8 +193,9 @@ enum Passed : int { PASSED = 0, LOST = 1, FAILED = -1 };
 // other opcode, so their fall-through (failure, particle lost, as for an
 // unknown type id) is never taken.  Maps that cannot lose a particle return a
 // constant, so the walk tests nothing after them.  OWN: drifts and multipoles
-// are the walk's (own_loop).
-template <bool FAST, int KIND, bool S_LIVE, bool DENSE, bool OWN>
+// are the walk's (own_loop).  EBE: the state need not be 1; an aperture leaves
+// its lowest bit (state &= inside in the reference).
+template <bool FAST, int KIND, bool S_LIVE, bool EBE, bool DENSE, bool OWN>
 __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t hdr,
                                         const TrackParams &prm, const Recip &inv, int64_t start_elem,
                                         int64_t ord)
@@ -202,6 +203,7 @@ __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t
     uint32_t const op = (uint32_t)(hdr & 0xFF);
     uint32_t const aux = (uint32_t)(hdr >> 32);
     auto limit = [&](bool inside) {
+        if (EBE) p.state &= 1;
         if (inside) return PASSED;
         p.state = 0;
         return LOST;
@@ -210,7 +212,8 @@ __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t
     case OP_DRIFT:
         if constexpr (OWN) break;
         drift<FAST, S_LIVE, DENSE>(p, W(rec[1]));
-        return limit(!(aux & DRIFT_APERTURE) || inside_global(p, prm.xlim_bits, prm.ylim_bits));
+        if (!(aux & DRIFT_APERTURE)) return PASSED;
+        return limit(inside_global(p, prm.xlim_bits, prm.ylim_bits));
     case OP_MULTIPOLE:
         if constexpr (OWN) break;
         multipole<FAST, false, KIND != KIND_SIMPLE, DENSE>(p, rec, aux);
@@ -232,7 +235,8 @@ __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t
         return PASSED;
     case OP_DRIFT_EXACT:
         drift_exact<S_LIVE>(p, W(rec[1]));
-        return limit(!(aux & DRIFT_APERTURE) || inside_global(p, prm.xlim_bits, prm.ylim_bits));
+        if (!(aux & DRIFT_APERTURE)) return PASSED;
+        return limit(inside_global(p, prm.xlim_bits, prm.ylim_bits));
     case OP_LIMIT_RECT:
         return limit(inside_rect(p, rec));
     case OP_LIMIT_RECT_ELLIPSE:
@@ -405,7 +409,8 @@ __device__ __forceinline__ void walk_chunk(PState &p, const uint64_t *rec, const
                 store_record(p, prm.ebe_out, prm.ebe_cap, j, ae, p.at_turn,
                              p.lazy_s ? prm.s_table[first + o] : p.s);
         }
-        Passed const rc = apply<FAST, KIND, S_LIVE, DENSE, kOwn>(p, rec, hdr, prm, inv, start_elem, first + o);
+        Passed const rc = apply<FAST, KIND, S_LIVE, EBE, DENSE, kOwn>(p, rec, hdr, prm, inv,
+                                                                       start_elem, first + o);
         if (rc != PASSED || (EBE && p.state != 1)) return stop(rc);
         ++o;
         rec = next;
