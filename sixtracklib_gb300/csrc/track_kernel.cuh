@@ -295,8 +295,12 @@ __device__ __forceinline__ Passed apply(PState &p, const uint64_t *rec, uint64_t
         }
     case OP_TRICUB:
         if constexpr (KIND == KIND_FULL) {
+            int64_t const state = p.state;
+            if (EBE) p.state = 1;
             p = tricub_element<FAST>(p, rec, aux);
-            return p.state == 1 ? PASSED : FAILED;  // outside the grid: lost, failure
+            if (p.state != 1) return FAILED;  // outside the grid: lost, failure
+            if (EBE) p.state = state;
+            return PASSED;
         } else if constexpr (KIND == KIND_MAP) {
             GridKick const k = tricub<FAST>(p.px, p.py, p.zeta, p.beta0, p.rvv,
                                             p.q0 * p.charge_ratio, p.p0c, p.x, p.y, rec, aux);

@@ -47,7 +47,7 @@ def lattice(kind, data=None):
 
 
 @pytest.mark.parametrize("kind", ["drift", "exact drift", "rect", "ellipse", "rect ellipse",
-                                  "multipole", "tricub"])
+                                  "multipole", "tricub", "tricub and beams"])
 def test_states_like_the_oracle(kind):
     e = lattice(kind)
     n = 40 * len(STATES)
