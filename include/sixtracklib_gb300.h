@@ -779,8 +779,9 @@ void st_TrackJobNew_set_collect_flags(st_TrackJobBaseNew *job, uint16_t flags);
 bool st_TrackJobNew_is_collecting_particles(const st_TrackJobBaseNew *job);
 void st_TrackJobNew_enable_collect_particles(st_TrackJobBaseNew *job);
 void st_TrackJobNew_disable_collect_particles(st_TrackJobBaseNew *job);
-/* cuda/track_job.h: the tracking kernel's largest block size (the one it runs
- * with where it is configured), and the configured threads_per_block. */
+/* cuda/track_job.h: the tracking kernel's block size as it runs over the job's
+ * particles (once some are lost, a launch over the others may take a smaller
+ * one unless it is configured), and the configured threads_per_block. */
 uint64_t st_CudaTrackJob_default_track_threads_per_block(const st_CudaTrackJob *job);
 uint64_t st_CudaTrackJob_default_threads_per_block(const st_CudaTrackJob *job);
 

@@ -2163,7 +2163,11 @@ void st_TrackJobNew_disable_collect_particles(st_TrackJobBaseNew *j)
 }
 uint64_t st_CudaTrackJob_default_track_threads_per_block(const st_CudaTrackJob *j)
 {
-    return j ? (uint64_t)j->opt.threads : 0;
+    if (!j) return 0;
+    if (j->opt.threads_given || !j->lat) return (uint64_t)j->opt.threads;
+    auto const &info = j->lat->cs.info;
+    return (uint64_t)default_track_threads(j->n_total, info.num_chunks, j->opt.stages,
+                                           info.chunk_words);
 }
 uint64_t st_CudaTrackJob_default_threads_per_block(const st_CudaTrackJob *j)
 {

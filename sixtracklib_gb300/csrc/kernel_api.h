@@ -76,9 +76,13 @@ struct TrackParams {
     uint32_t op_mask;        // opcodes present in the compiled range (stream.h)
 };
 
+// Threads per block of a launch over `count` particles where the caller gives
+// none.
+int default_track_threads(int64_t count, int n_chunks, int stages, int chunk_words);
+
 // Launch one tracking kernel on `stream` (a cudaStream_t).  Returns the CUDA
 // error code of the launch (0 on success).
-// threads 0: chosen by the number of particles.
+// threads 0: default_track_threads.
 // blocks_per_sm selects the register tier: 1 (up to 255 registers, no
 // spills) or 2 (at most 128 registers per thread, two CTAs per SM).
 // prm.op_mask selects the instantiation (lattice_kind).

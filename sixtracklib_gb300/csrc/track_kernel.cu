@@ -64,8 +64,9 @@ size_t track_smem_bytes(int stages, int chunk_words)
 // (64 / 128) 1.54 / 1.66; 2,000-element ring, exact, 131,072 3.28 / 3.33.
 // Three stages of 8 KiB let nine blocks reside, four only six (131,072: 64
 // threads 4.03 ms).
-static int default_threads(int64_t count, size_t smem)
+int default_track_threads(int64_t count, int n_chunks, int stages, int chunk_words)
 {
+    size_t const smem = track_smem_bytes(std::min(n_chunks, stages), chunk_words);
     int64_t const blocks = (int64_t)((228u << 10) / (smem + 1152u));
     int64_t const wanted = std::min<int64_t>((count + 151) / 152, 512);
     for (int threads : {32, 64})
@@ -83,7 +84,7 @@ int launch_track(const TrackParams &params, bool fast, int threads, int blocks_p
     if (prm.n_chunks < prm.stages) prm.stages = prm.n_chunks;
     size_t const smem = track_smem_bytes(prm.stages, prm.chunk_words);
     if (threads <= 0)
-        threads = default_threads(count, smem);
+        threads = default_track_threads(count, prm.n_chunks, prm.stages, prm.chunk_words);
     else if (threads > kMaxThreads || threads % 32 != 0)
         threads = kMaxThreads;
     unsigned const blocks = (unsigned)((count + threads - 1) / threads);
