@@ -10,7 +10,7 @@
 // momentum and where the sums agree they are the FP64 evaluation's, else it
 // is run.  Gaussian profiles (q = 1) only.  One turn of the FODO ring with 200
 // such kicks and 4 + 4 beam-beam elements, fast: round beams, 65,536
-// protons, 2 turns 5.18 -> 3.24 ms; elliptic, 33,333 protons 13.3 -> 8.6 ms
+// protons, 2 turns 5.05 -> 3.24 ms; elliptic, 33,333 protons 13.3 -> 8.6 ms
 // (100,000: 41.6 -> 19.7 ms).
 //
 // The Faddeeva function follows faddeeva_cern.h:45-120 in the form of
@@ -25,85 +25,43 @@
 
 namespace stg {
 
-// 2^(j / 32) as pairs of floats
+// 2^(j / 32) as pairs of floats: h the nearest float, l the nearest float of
+// the rest (from 60 decimal digits).  An entry is read in one load of 8 bytes,
+// which an array of floats is not aligned for.
+struct alignas(8) ExpPair {
+    float h, l;
+};
+#define STG_EXP32                                                           \
+    {0x1p+0f, 0.0f}, {0x1.059b0ep+0f, -0x1.9d4f52p-25f},                    \
+    {0x1.0b5586p+0f, 0x1.9f3122p-25f}, {0x1.11301ep+0f, -0x1.fdb496p-25f},  \
+    {0x1.172b84p+0f, -0x1.c15742p-27f}, {0x1.1d4874p+0f, -0x1.d2e8cap-25f}, \
+    {0x1.2387a6p+0f, 0x1.ceac48p-25f}, {0x1.29e9ep+0f, -0x1.5c0424p-25f},   \
+    {0x1.306fep+0f, 0x1.4636e2p-25f}, {0x1.371a74p+0f, -0x1.18aac6p-25f},   \
+    {0x1.3dea64p+0f, 0x1.824684p-25f}, {0x1.44e086p+0f, 0x1.8624b4p-30f},   \
+    {0x1.4bfdaep+0f, -0x1.593abcp-25f}, {0x1.5342b6p+0f, -0x1.2c561p-25f},  \
+    {0x1.5ab07ep+0f, -0x1.5bd5ecp-27f}, {0x1.6247ecp+0f, -0x1.f8b55p-25f},  \
+    {0x1.6a09e6p+0f, 0x1.9fcef4p-26f}, {0x1.71f75ep+0f, 0x1.1d8beep-25f},   \
+    {0x1.7a1148p+0f, -0x1.829fdp-25f}, {0x1.82589ap+0f, -0x1.accc7cp-26f},  \
+    {0x1.8ace54p+0f, 0x1.15506ep-27f}, {0x1.93737cp+0f, -0x1.e64744p-25f},  \
+    {0x1.9c4918p+0f, 0x1.51f848p-27f}, {0x1.a5503cp+0f, -0x1.b83b54p-25f},  \
+    {0x1.ae89fap+0f, -0x1.a94b14p-26f}, {0x1.b7f77p+0f, -0x1.a09438p-25f},  \
+    {0x1.c199bep+0f, -0x1.3d56b2p-27f}, {0x1.cb720ep+0f, -0x1.8837ccp-27f}, \
+    {0x1.d5818ep+0f, -0x1.822dbcp-27f}, {0x1.dfc974p+0f, -0x1.908c94p-25f}, \
+    {0x1.ea4afap+0f, 0x1.52486cp-27f}, {0x1.f50766p+0f, -0x1.246ebp-26f}
+
 #if defined(__CUDACC__)
-static __device__ const float kExp32Dev[32][2] = {
-    {0x1.0000000000000p+0f, 0x0.0p+0f},
-    {0x1.059b0e0000000p+0f, -0x1.9d4f520000000p-25f},
-    {0x1.0b55860000000p+0f, 0x1.9f31220000000p-25f},
-    {0x1.11301e0000000p+0f, -0x1.fdb4960000000p-25f},
-    {0x1.172b840000000p+0f, -0x1.c157420000000p-27f},
-    {0x1.1d48740000000p+0f, -0x1.d2e8ca0000000p-25f},
-    {0x1.2387a60000000p+0f, 0x1.ceac480000000p-25f},
-    {0x1.29e9e00000000p+0f, -0x1.5c04240000000p-25f},
-    {0x1.306fe00000000p+0f, 0x1.4636e20000000p-25f},
-    {0x1.371a740000000p+0f, -0x1.18aac60000000p-25f},
-    {0x1.3dea640000000p+0f, 0x1.8246840000000p-25f},
-    {0x1.44e0860000000p+0f, 0x1.8624b40000000p-30f},
-    {0x1.4bfdae0000000p+0f, -0x1.593abc0000000p-25f},
-    {0x1.5342b60000000p+0f, -0x1.2c56100000000p-25f},
-    {0x1.5ab07e0000000p+0f, -0x1.5bd5ec0000000p-27f},
-    {0x1.6247ec0000000p+0f, -0x1.f8b5500000000p-25f},
-    {0x1.6a09e60000000p+0f, 0x1.9fcef40000000p-26f},
-    {0x1.71f75e0000000p+0f, 0x1.1d8bee0000000p-25f},
-    {0x1.7a11480000000p+0f, -0x1.829fd00000000p-25f},
-    {0x1.82589a0000000p+0f, -0x1.accc7c0000000p-26f},
-    {0x1.8ace540000000p+0f, 0x1.15506e0000000p-27f},
-    {0x1.93737c0000000p+0f, -0x1.e647440000000p-25f},
-    {0x1.9c49180000000p+0f, 0x1.51f8480000000p-27f},
-    {0x1.a5503c0000000p+0f, -0x1.b83b540000000p-25f},
-    {0x1.ae89fa0000000p+0f, -0x1.a94b140000000p-26f},
-    {0x1.b7f7700000000p+0f, -0x1.a094380000000p-25f},
-    {0x1.c199be0000000p+0f, -0x1.3d56b20000000p-27f},
-    {0x1.cb720e0000000p+0f, -0x1.8837cc0000000p-27f},
-    {0x1.d5818e0000000p+0f, -0x1.822dbc0000000p-27f},
-    {0x1.dfc9740000000p+0f, -0x1.908c940000000p-25f},
-    {0x1.ea4afa0000000p+0f, 0x1.52486c0000000p-27f},
-    {0x1.f507660000000p+0f, -0x1.246eb00000000p-26f},
-};
+static __device__ const ExpPair kExp32Dev[32] = {STG_EXP32};
 #endif
-static const float kExp32[32][2] = {
-    {0x1.0000000000000p+0f, 0x0.0p+0f},
-    {0x1.059b0e0000000p+0f, -0x1.9d4f520000000p-25f},
-    {0x1.0b55860000000p+0f, 0x1.9f31220000000p-25f},
-    {0x1.11301e0000000p+0f, -0x1.fdb4960000000p-25f},
-    {0x1.172b840000000p+0f, -0x1.c157420000000p-27f},
-    {0x1.1d48740000000p+0f, -0x1.d2e8ca0000000p-25f},
-    {0x1.2387a60000000p+0f, 0x1.ceac480000000p-25f},
-    {0x1.29e9e00000000p+0f, -0x1.5c04240000000p-25f},
-    {0x1.306fe00000000p+0f, 0x1.4636e20000000p-25f},
-    {0x1.371a740000000p+0f, -0x1.18aac60000000p-25f},
-    {0x1.3dea640000000p+0f, 0x1.8246840000000p-25f},
-    {0x1.44e0860000000p+0f, 0x1.8624b40000000p-30f},
-    {0x1.4bfdae0000000p+0f, -0x1.593abc0000000p-25f},
-    {0x1.5342b60000000p+0f, -0x1.2c56100000000p-25f},
-    {0x1.5ab07e0000000p+0f, -0x1.5bd5ec0000000p-27f},
-    {0x1.6247ec0000000p+0f, -0x1.f8b5500000000p-25f},
-    {0x1.6a09e60000000p+0f, 0x1.9fcef40000000p-26f},
-    {0x1.71f75e0000000p+0f, 0x1.1d8bee0000000p-25f},
-    {0x1.7a11480000000p+0f, -0x1.829fd00000000p-25f},
-    {0x1.82589a0000000p+0f, -0x1.accc7c0000000p-26f},
-    {0x1.8ace540000000p+0f, 0x1.15506e0000000p-27f},
-    {0x1.93737c0000000p+0f, -0x1.e647440000000p-25f},
-    {0x1.9c49180000000p+0f, 0x1.51f8480000000p-27f},
-    {0x1.a5503c0000000p+0f, -0x1.b83b540000000p-25f},
-    {0x1.ae89fa0000000p+0f, -0x1.a94b140000000p-26f},
-    {0x1.b7f7700000000p+0f, -0x1.a094380000000p-25f},
-    {0x1.c199be0000000p+0f, -0x1.3d56b20000000p-27f},
-    {0x1.cb720e0000000p+0f, -0x1.8837cc0000000p-27f},
-    {0x1.d5818e0000000p+0f, -0x1.822dbc0000000p-27f},
-    {0x1.dfc9740000000p+0f, -0x1.908c940000000p-25f},
-    {0x1.ea4afa0000000p+0f, 0x1.52486c0000000p-27f},
-    {0x1.f507660000000p+0f, -0x1.246eb00000000p-26f},
-};
+static const ExpPair kExp32[32] = {STG_EXP32};
+#undef STG_EXP32
 
 STG_HD FPair exp32(int j)
 {
 #if defined(__CUDA_ARCH__)
-    float2 const v = __ldg(reinterpret_cast<const float2 *>(&kExp32Dev[j][0]));
+    float2 const v = __ldg(reinterpret_cast<const float2 *>(&kExp32Dev[j]));
     return FPair{v.x, v.y};
 #else
-    return FPair{kExp32[j][0], kExp32[j][1]};
+    return FPair{kExp32[j].h, kExp32[j].l};
 #endif
 }
 

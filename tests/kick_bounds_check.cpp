@@ -218,13 +218,27 @@ static void tails(bool round, long n, long *undecided, long *different)
     }
 }
 
+// The table of exp_pair: entries and their alignment for one load each.
+static void table(long *different)
+{
+    for (int j = 0; j < 32; ++j) {
+        long double const v = exp2l(j / 32.0L);
+        float const h = (float)v, l = (float)(v - h);
+        FPair const t = exp32(j);
+        if (t.h != h || t.l != l || alignof(decltype(kExp32[0])) < 8 || (uintptr_t)&kExp32[j] % 8)
+            ++*different;
+    }
+}
+
 int main(int argc, char **argv)
 {
     if (argc < 4) return 2;
     long const n = atol(argv[2]);
     gen.seed((uint64_t)atol(argv[3]));
     long undecided = 0, different = 0;
-    if (!strcmp(argv[1], "near axis"))
+    if (!strcmp(argv[1], "table"))
+        table(&different);
+    else if (!strcmp(argv[1], "near axis"))
         near_axis(n, &undecided, &different);
     else if (!strncmp(argv[1], "tails", 5))
         tails(!strcmp(argv[1], "tails round"), n, &undecided, &different);

@@ -52,3 +52,8 @@ def test_space_charge_bounds_over_the_bunch(check, beam):
     print(f"{beam}: {undecided} of {n} left to the FP64 evaluation")
     assert different == 0
     assert undecided < n
+
+
+def test_exponential_table(check):
+    """Its entries, and their alignment for a load of 8 bytes."""
+    assert check("table", 32, 0) == [32, 0, 0]
