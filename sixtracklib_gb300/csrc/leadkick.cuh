@@ -117,8 +117,11 @@ STG_HD double as_double(float v)
     return a < 0x00800000u ? 0.0 : from_words(((a >> 3) + 0x38000000u) | (w & 0x80000000u), w << 29);
 }
 
-// Doubles at or outside both ends of [h + l - d, h + l + d] (d with a slack
-// of a unit in their last place).
+// Doubles at or outside both ends of [h + l - d, h + l + d].  l is up to 2^28
+// units of the last of h's 53 bits and l -+ d is rounded to 24 bits, so d has to
+// hold 8 such units (2^-49 of h) more than the error it bounds: the 5 % that
+// lead_block adds to bounds of 2^-43 and more do, as does what sc_pair_kick's
+// bound leaves over.
 STG_HD void double_bounds(FPair v, float d, double *lo_v, double *hi_v)
 {
     float const h = fadd(v.h, v.l), l = fsub(v.l, fsub(h, v.h));

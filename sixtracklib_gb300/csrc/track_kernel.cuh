@@ -438,9 +438,10 @@ __device__ __forceinline__ void mbar_inval(uint64_t *bar)
 constexpr int64_t kDenseParticles = 2 * 32 * 4 * 152;
 
 // One CTA's share of a tracking call: particle t of the launch (an index
-// into prm.idx, or prm.i0 + t).  Block-uniform control flow: every thread
-// walks every record of every chunk of every turn the block needs; lanes
-// whose particle is done are predicated off inside apply().  `smem` holds
+// into prm.idx, or prm.i0 + t).  The loops over turns and chunks are
+// block-uniform; within a chunk only lanes whose particle takes part walk its
+// records, and one whose particle stops leaves the walk (walk_chunk), all of
+// them back together at the barrier after the chunk or the turn.  `smem` holds
 // 16 words of mbarriers followed by prm.stages chunk buffers.  Returns with
 // every copy it issued complete; the caller invalidates the barriers before
 // the shared memory is used again.
